@@ -243,14 +243,14 @@ int psm_adjoint_device(psm_ctx *ctx, const float *d_image, float *d_data);
  * traces. */
 int psm_lsm_cg(psm_ctx *ctx, const float *data, float *image, int iters, double *resid);
 
-/* Forward-kernel variants: f32x2-packed or scalar FP32 arithmetic for each pair of 32-sample
- * blocks, 2, 4 or 8 blocks behind one warp-uniform skip test, and 8 or 16 blocks per lane (a
- * tile of 256 or 512 output samples).  All give the same masks and the same terms, bit for
- * bit; they differ in instruction count and shared-memory traffic.  The PAIRS variants (fp32
- * storage) evaluate the travel time once for the two traces at inlines c - d and c + d of one
- * crossline, which share it, and add their two samples before the weight: the same terms,
- * summed in another order (equal to FP32 rounding).  PSM_FWD_DEFAULT lets the
- * library pick (the result of psm_autotune once it has run on the ctx). */
+/* Forward-kernel variants.  There are two kernels, which differ in the output crosslines of a
+ * tile: 14 (wide tiles) and 4 (narrow tiles, for problems whose wide tiles do not fill the
+ * GPU).  Both evaluate the travel time once for the two traces at inlines c - d and c + d of
+ * one crossline, which share it; they give the same terms under the same masks and differ in
+ * the order in which an output sample's terms are added (equal to FP32 rounding).
+ * PSM_FWD_PAIRS and PSM_FWD_PAIRS_J4_O4 run the narrow tiles, every other id the wide ones (the
+ * ids of earlier kernels are kept).  PSM_FWD_DEFAULT chooses by the problem's size (until
+ * psm_autotune has run on the ctx, whose result it then is). */
 typedef enum {
     PSM_FWD_DEFAULT = 0,
     PSM_FWD_SCALAR_G2 = 1,
@@ -261,18 +261,18 @@ typedef enum {
     PSM_FWD_SCALAR_G4_J16 = 6,
     PSM_FWD_PACKED_G8 = 7,
     PSM_FWD_SCALAR_G8 = 8,
-    PSM_FWD_PACKED_G4_O3 = 9,  /* 3 CTAs per SM: 72 registers, 32 KB stages */
+    PSM_FWD_PACKED_G4_O3 = 9,
     PSM_FWD_SCALAR_G4_O3 = 10,
-    PSM_FWD_PAIRS_O3 = 11, /* mirrored inlines c - d, c + d staged as pairs, 3 CTAs per SM */
-    PSM_FWD_PAIRS = 12,
-    PSM_FWD_PAIRS_J4_O4 = 13, /* pairs, tiles of 128 samples, 4 CTAs per SM (56 registers) */
+    PSM_FWD_PAIRS_O3 = 11,    /* wide tiles */
+    PSM_FWD_PAIRS = 12,       /* narrow tiles */
+    PSM_FWD_PAIRS_J4_O4 = 13, /* narrow tiles */
     PSM_FWD_N_VARIANTS = 14
 } psm_fwd_variant;
 int psm_set_variant(psm_ctx *ctx, int variant);
 int psm_get_variant(psm_ctx *ctx, int *variant);
-/* Time one forward launch of every variant on the resident cube (CUDA events on the ctx
- * stream), keep the fastest for this ctx.  ms[PSM_FWD_N_VARIANTS] (may be NULL) receives the
- * times, ms[0] unused; *best (may be NULL) the chosen variant. */
+/* Time one forward launch of each kernel on the resident cube (CUDA events on the ctx
+ * stream), keep the fastest for this ctx.  ms[PSM_FWD_N_VARIANTS] (may be NULL) receives every
+ * variant's kernel's time, ms[0] unused; *best (may be NULL) the chosen variant. */
 int psm_autotune(psm_ctx *ctx, float *ms, int *best);
 
 /* Number of (output sample, input trace) terms that pass every mask of the reference
@@ -333,11 +333,11 @@ typedef enum {
 } psm_tile_order;
 int psm_batch_set_order(psm_batch *batch, int order);
 int psm_batch_get_order(psm_batch *batch, int *order);
-/* Times one run per distinct kernel variant on each of five schedules (0 persistent
+/* Times one run of each kernel on each of five schedules (0 persistent
  * depth-first, 1 persistent problem order, 2 one launch per problem, 3 one grid depth-first,
  * 4 one grid problem order) and keeps the fastest
  * variant, order and mode; ms[5 * PSM_FWD_N_VARIANTS] (may be NULL) receives the times at
- * [schedule * PSM_FWD_N_VARIANTS + variant], 0 for variants not run. */
+ * [schedule * PSM_FWD_N_VARIANTS + variant], 0 for ids that stand for another. */
 int psm_batch_autotune(psm_batch *batch, float *ms, int *best, int *best_order,
                        int *best_mode);
 int psm_batch_run_async(psm_batch *batch); /* on the context's stream */

@@ -27,8 +27,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 # translation units of libpsm_cuda.so, compiled in parallel and linked into one library
 CUDA_SRC = [os.path.join(CSRC, "psm_cuda.cu"), os.path.join(CSRC, "psm_limbs.cu")]
-CUDA_HDR = [os.path.join(CSRC, h) for h in ("psm_kernels.cuh", "psm_adjoint.cuh",
-                                             "psm_segy.cuh", "psm_vrms.cuh")] + \
+CUDA_HDR = [os.path.join(CSRC, h) for h in ("psm_kernels.cuh", "psm_forward.cuh",
+                                             "psm_adjoint.cuh", "psm_segy.cuh",
+                                             "psm_vrms.cuh")] + \
     [os.path.join(INC, "psm.h")]
 CUDA_DEPS = CUDA_SRC + CUDA_HDR
 # Flush-to-zero: the reference's -ffast-math build runs with FTZ/DAZ set (GCC links

@@ -24,6 +24,12 @@
 
 namespace psm {
 
+constexpr int kTX = 8;          // output crosslines per CTA (one consumer warp each)
+constexpr int kJ = 8;           // 32-sample blocks per consumer lane
+constexpr int kTT = 32 * kJ;    // output samples per CTA
+constexpr int kMaxG = 32;       // traces per ring stage
+static_assert(kTX % 4 == 0, "per-slot r^2 rows are stored as float4");
+
 struct AdjParams {
     FwdParams F;          // geometry, tables, constants (F.pairs unused)
     const float* image;   // [n_jobs][n_ox][n_t]: image of each job (duplicate rows folded)

@@ -17,6 +17,7 @@
 
 #include "psm.h"
 #include "psm_adjoint.cuh"
+#include "psm_forward.cuh"
 #include "psm_kernels.cuh"
 #include "psm_segy.cuh"
 #include "psm_vrms.cuh"
@@ -28,14 +29,19 @@ using psm::Job;
 
 constexpr size_t kMaxDynSmem = 232448;  // 227 KB per CTA on sm_100
 
-// Trace stride in HBM: n_t rounded up to 8 samples so every trace starts 32 B aligned for
-// the TMA bulk copies; the tail samples stay zero.
-inline int trace_stride(int n_t) { return (n_t + 7) & ~7; }
+// Trace stride in HBM: a multiple of 8 samples above n_t, so that every trace starts 16 B
+// aligned for the TMA bulk copies (in 16-bit storage too) and ends in a zero sample.
+inline int trace_stride(int n_t) { return (n_t + 8) & ~7; }
 
-// Ring stage capacity (samples): 48 KB a stage, and at least one whole trace so a stage
-// always takes a window.
-inline int stage_cap(int ns, int store = psm::kStoreF32) {
-    return std::max(psm::kStageCapMin * 8 / psm::store_bytes(store), ns);
+// Largest problems the entry points take: two staging buffers of at least one whole trace
+// (elem_bytes a sample) and 12 bytes an inline of the widest buffer in one CTA's shared memory.
+// The forward kernel itself needs less (a window longer than a stage is staged in parts); the
+// adjoint stages whole windows.
+inline bool fits_staging(int64_t max_inl, int n_t, int elem_bytes) {
+    const int64_t ns = (int64_t(n_t) + 7) & ~int64_t(7);
+    const int64_t cap = std::max<int64_t>(6144 * 8 / elem_bytes, ns);
+    const int64_t tables = (4096 + 12 * max_inl + 4 + 127) & ~int64_t(127);
+    return tables + 2 * elem_bytes * cap + 128 <= int64_t(kMaxDynSmem);
 }
 
 // Storage of a geometry's traces (psm_precision -> psm::kStore*).
@@ -47,6 +53,17 @@ inline int store_of(int precision) {
 int max_inline_window(const std::vector<Job>& jobs) {
     int m = 1;
     for (const Job& j : jobs) m = std::max(m, j.i1 - j.i0);
+    return m;
+}
+
+// Rows of a job's trace list when inline positions are consecutive: mirror distances from its
+// own inline (buffer inline `c`), or every inline when it lies outside the buffer.
+inline int list_rows(int c, int n_inl) {
+    return c >= 0 && c < n_inl ? std::max(c, n_inl - 1 - c) + 1 : std::max(n_inl, 1);
+}
+int max_list_rows(const std::vector<Job>& jobs) {
+    int m = 1;
+    for (const Job& j : jobs) m = std::max(m, list_rows(j.pos - j.i0, j.i1 - j.i0));
     return m;
 }
 
@@ -102,185 +119,107 @@ struct Status {
                              std::string(#call) + ": " + cudaGetErrorString(e_));        \
     } while (0)
 
-// Dynamic shared memory of a forward launch (0: too large for one CTA).
-size_t fwd_smem(const FwdParams& P, int store = psm::kStoreF32) {
-    const size_t b = psm::smem_layout(P.max_inl, P.stage_cap, psm::store_bytes(store)).total;
-    return b <= kMaxDynSmem ? b : 0;
-}
-
+// ---- forward kernel variants (psm_fwd_variant).  Two kernels: tiles of 14 output crosslines
+// for 2 CTAs per SM, and tiles of 4 crosslines for 3, for problems whose wide tiles do not fill
+// the GPU.  PSM_FWD_PAIRS and PSM_FWD_PAIRS_J4_O4 name the narrow tiles, every other id the wide
+// ones.
 constexpr int kDefaultVariant = PSM_FWD_PAIRS_O3;
 
-inline bool is_j16(int variant) {
-    return variant == PSM_FWD_PACKED_G4_J16 || variant == PSM_FWD_SCALAR_G4_J16;
-}
-
-inline bool is_o3(int variant) {
-    return variant == PSM_FWD_PACKED_G4_O3 || variant == PSM_FWD_SCALAR_G4_O3 ||
-           variant == PSM_FWD_PAIRS_O3;
-}
-
-inline bool is_pairs(int variant) {
-    return variant == PSM_FWD_PAIRS_O3 || variant == PSM_FWD_PAIRS;
-}
-
-// The variant that actually runs: 16-bit storage and compensated summation run the packed
-// skip-4 kernel, with 16 blocks a lane (16-bit storage only: compensation's partial and
-// compensation registers leave no room for 16), or built for 3 CTAs per SM, each with or
-// without mirrored pairs.
+// The variant id a request stands for: 16-bit storage and compensated summation know five ids.
 inline int effective_variant(int variant, int store, bool kahan) {
     if (variant == PSM_FWD_DEFAULT) variant = kDefaultVariant;
     if (store == psm::kStoreF32 && !kahan) return variant;
-    if (!kahan && is_j16(variant)) return PSM_FWD_PACKED_G4_J16;
-    if (is_pairs(variant)) return variant;
-    return is_o3(variant) ? PSM_FWD_PACKED_G4_O3 : PSM_FWD_PACKED_G4;
+    const bool j16 = variant == PSM_FWD_PACKED_G4_J16 || variant == PSM_FWD_SCALAR_G4_J16;
+    if (!kahan && j16) return PSM_FWD_PACKED_G4_J16;
+    if (variant == PSM_FWD_PAIRS_O3 || variant == PSM_FWD_PAIRS) return variant;
+    return variant == PSM_FWD_PACKED_G4_O3 || variant == PSM_FWD_SCALAR_G4_O3
+               ? PSM_FWD_PACKED_G4_O3
+               : PSM_FWD_PACKED_G4;
 }
 
-// One instantiation of the forward kernel templates (MINB: CTAs per SM the kernel is built
-// for, 2 or 3).
-template <bool AMP_, bool PACKED_, int GB_, int J_, int STORE_, bool KAHAN_, int MINB_ = 2,
-          bool PAIRS_ = false>
+// One instantiation of the forward kernel templates (ORDERED: terms in trace order, grid
+// launches only; NX crosslines a tile, CAP samples a stage, MINB CTAs per SM).
+template <bool AMP_, bool KAHAN_, bool ORDERED_, int NX_, int CAP_, int MINB_>
 struct KernelTag {
-    static constexpr bool AMP = AMP_, PACKED = PACKED_, KAHAN = KAHAN_, PAIRS = PAIRS_;
-    static constexpr int GB = GB_, J = J_, STORE = STORE_, MINB = MINB_;
+    static constexpr bool AMP = AMP_, KAHAN = KAHAN_, ORDERED = ORDERED_;
+    static constexpr int NX = NX_, CAP = CAP_, MINB = MINB_;
+    using Layout = psm::FwdLayout<NX_, CAP_>;
+    static constexpr int threads = 32 * (NX_ + 2);
 };
+constexpr int kWideNX = 14, kNarrowNX = 4;
 
-// Samples per stage of the kernel built for 3 CTAs per SM (32 KB) or 4 (20 KB), so that its
-// shared memory fits the SM three or four times.
-inline int stage_cap_for(int minb, int store) {
-    return psm::stage_bytes_for(minb) / psm::store_bytes(store);
+template <bool AMP, bool KAHAN, bool ORDERED>
+using WideTag = KernelTag<AMP, KAHAN, ORDERED, kWideNX, 4096, 2>;
+template <bool AMP, bool KAHAN, bool ORDERED>
+using NarrowTag = KernelTag<AMP, KAHAN, ORDERED, kNarrowNX, 2432, 3>;
+
+// Narrow tiles for a problem whose wide tiles do not fill the SMs (launches of a few jobs of a
+// larger problem keep the problem's tiles, so that their images are the same bit for bit).
+inline bool few_tiles(int64_t n_jobs, int n_ox, int n_t) {
+    return n_jobs * ((n_ox + kWideNX - 1) / kWideNX) * ((n_t + psm::kTileT - 1) / psm::kTileT) <
+           148;
+}
+// Whether `variant` runs narrow tiles (`few`: the problem's own choice, taken by the default).
+inline bool narrow_tiles(int variant, int store, bool kahan, bool few) {
+    if (variant == PSM_FWD_DEFAULT) return few;
+    const int v = effective_variant(variant, store, kahan);
+    return v == PSM_FWD_PAIRS || v == PSM_FWD_PAIRS_J4_O4;
+}
+
+// Calls f(KernelTag<...>{}) for the kernel that (amp, kahan, narrow) names.
+template <bool ORDERED = false, class F>
+cudaError_t with_kernel(bool amp, bool kahan, bool narrow, F&& f) {
+    if (narrow)
+        return amp ? (kahan ? f(NarrowTag<true, true, ORDERED>{})
+                            : f(NarrowTag<true, false, ORDERED>{}))
+                   : (kahan ? f(NarrowTag<false, true, ORDERED>{})
+                            : f(NarrowTag<false, false, ORDERED>{}));
+    return amp ? (kahan ? f(WideTag<true, true, ORDERED>{}) : f(WideTag<true, false, ORDERED>{}))
+               : (kahan ? f(WideTag<false, true, ORDERED>{}) : f(WideTag<false, false, ORDERED>{}));
 }
 
 template <class K>
 auto grid_kernel() {
-    if constexpr (K::MINB == 4)
-        return psm::fwd_kernel_o4<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN, K::PAIRS>;
-    else if constexpr (K::MINB == 3)
-        return psm::fwd_kernel_o3<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN, K::PAIRS>;
-    else
-        return psm::fwd_kernel<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN, K::PAIRS>;
+    return psm::fwd_kernel<K::AMP, K::KAHAN, K::ORDERED, K::NX, K::CAP, K::MINB>;
 }
 
-// Calls f(KernelTag<...>{}) for the kernel that (amp, effective variant, store, kahan) names.
-template <bool AMP, class F>
-cudaError_t with_kernel_amp(int variant, int store, bool kahan, F&& f) {
-    using psm::kStoreBF16;
-    using psm::kStoreF16;
-    using psm::kStoreF32;
-    const bool j16 = is_j16(variant), o3 = is_o3(variant), pr = is_pairs(variant);
-    // 16-bit storage or compensated summation with mirrored pairs
-    if (pr && (store != kStoreF32 || kahan)) {
-        switch (store * 2 + (kahan ? 1 : 0)) {
-#define PSM_PAIR_CASE(ST, KA)                                                                \
-    case ST * 2 + KA:                                                                        \
-        return o3 ? f(KernelTag<AMP, true, 4, 8, ST, KA, 3, true>{})                         \
-                  : f(KernelTag<AMP, true, 4, 8, ST, KA, 2, true>{});
-            PSM_PAIR_CASE(kStoreF32, 1)
-            PSM_PAIR_CASE(kStoreBF16, 0)
-            PSM_PAIR_CASE(kStoreBF16, 1)
-            PSM_PAIR_CASE(kStoreF16, 0)
-            PSM_PAIR_CASE(kStoreF16, 1)
-#undef PSM_PAIR_CASE
-            default: return cudaErrorInvalidValue;
-        }
-    }
-    switch (store * 2 + (kahan ? 1 : 0)) {
-        case kStoreF32 * 2:
-            switch (variant) {
-                case PSM_FWD_SCALAR_G2: return f(KernelTag<AMP, false, 2, 8, kStoreF32, false>{});
-                case PSM_FWD_SCALAR_G4: return f(KernelTag<AMP, false, 4, 8, kStoreF32, false>{});
-                case PSM_FWD_PACKED_G2: return f(KernelTag<AMP, true, 2, 8, kStoreF32, false>{});
-                case PSM_FWD_PACKED_G4: return f(KernelTag<AMP, true, 4, 8, kStoreF32, false>{});
-                case PSM_FWD_PACKED_G4_J16:
-                    return f(KernelTag<AMP, true, 4, 16, kStoreF32, false>{});
-                case PSM_FWD_SCALAR_G4_J16:
-                    return f(KernelTag<AMP, false, 4, 16, kStoreF32, false>{});
-                case PSM_FWD_PACKED_G8: return f(KernelTag<AMP, true, 8, 8, kStoreF32, false>{});
-                case PSM_FWD_SCALAR_G8: return f(KernelTag<AMP, false, 8, 8, kStoreF32, false>{});
-                case PSM_FWD_PACKED_G4_O3:
-                    return f(KernelTag<AMP, true, 4, 8, kStoreF32, false, 3>{});
-                case PSM_FWD_SCALAR_G4_O3:
-                    return f(KernelTag<AMP, false, 4, 8, kStoreF32, false, 3>{});
-                case PSM_FWD_PAIRS_O3:
-                    return f(KernelTag<AMP, true, 4, 8, kStoreF32, false, 3, true>{});
-                case PSM_FWD_PAIRS: return f(KernelTag<AMP, true, 4, 8, kStoreF32, false, 2, true>{});
-                case PSM_FWD_PAIRS_J4_O4:
-                    return f(KernelTag<AMP, true, 4, 4, kStoreF32, false, 4, true>{});
-
-
-                default: return cudaErrorInvalidValue;
-            }
-        case kStoreF32 * 2 + 1:
-            return o3 ? f(KernelTag<AMP, true, 4, 8, kStoreF32, true, 3>{})
-                      : f(KernelTag<AMP, true, 4, 8, kStoreF32, true>{});
-        case kStoreBF16 * 2:
-            return j16  ? f(KernelTag<AMP, true, 4, 16, kStoreBF16, false>{})
-                   : o3 ? f(KernelTag<AMP, true, 4, 8, kStoreBF16, false, 3>{})
-                        : f(KernelTag<AMP, true, 4, 8, kStoreBF16, false>{});
-        case kStoreBF16 * 2 + 1:
-            return o3 ? f(KernelTag<AMP, true, 4, 8, kStoreBF16, true, 3>{})
-                      : f(KernelTag<AMP, true, 4, 8, kStoreBF16, true>{});
-        case kStoreF16 * 2:
-            return j16  ? f(KernelTag<AMP, true, 4, 16, kStoreF16, false>{})
-                   : o3 ? f(KernelTag<AMP, true, 4, 8, kStoreF16, false, 3>{})
-                        : f(KernelTag<AMP, true, 4, 8, kStoreF16, false>{});
-        case kStoreF16 * 2 + 1:
-            return o3 ? f(KernelTag<AMP, true, 4, 8, kStoreF16, true, 3>{})
-                      : f(KernelTag<AMP, true, 4, 8, kStoreF16, true>{});
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-template <class F>
-cudaError_t with_kernel(bool amp, int variant, int store, bool kahan, F&& f) {
-    variant = effective_variant(variant, store, kahan);
-    return amp ? with_kernel_amp<true>(variant, store, kahan, f)
-               : with_kernel_amp<false>(variant, store, kahan, f);
-}
-
-// The grid kernel's shared-memory limit, set before a stream capture (the attribute belongs
-// to the kernel, so it must cover the largest launch of the capture).
-template <class K>
-cudaError_t prepare_grid(K, size_t smem) {
-    return cudaFuncSetAttribute(grid_kernel<K>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+// A kernel's shared-memory limit.  It belongs to the kernel, so before a stream capture it is
+// set to cover the largest launch of the capture.
+template <class Kernel>
+cudaError_t set_smem(Kernel* kern, size_t smem) {
+    if (smem > kMaxDynSmem) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(smem));
 }
 
 template <class K>
-cudaError_t launch_grid(K, const FwdParams& P_in, int n_jobs, size_t smem, cudaStream_t s) {
-    constexpr int TT = 32 * K::J;
+cudaError_t launch_grid(K, const FwdParams& P, int n_jobs, cudaStream_t s) {
     auto* kern = grid_kernel<K>();
-    FwdParams P = P_in;
-    if constexpr (K::MINB > 2) {  // smaller stages, so that MINB CTAs fit an SM
-        P.stage_cap = std::max(stage_cap_for(K::MINB, K::STORE), P.ns);
-        smem = std::min(smem, fwd_smem(P, K::STORE));
-    }
+    const size_t smem = K::Layout::total(P.store, P.max_rows);
     if (n_jobs > 65535) return cudaErrorInvalidValue;  // grid y
-    dim3 grid((P.n_ox + psm::kTX - 1) / psm::kTX, n_jobs, (P.n_t + TT - 1) / TT);
-    dim3 block(32 * (psm::kTX + 1));
+    dim3 grid((P.n_ox + K::NX - 1) / K::NX, n_jobs, (P.n_t + psm::kTileT - 1) / psm::kTileT);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &cap);
     if (e != cudaSuccess) return e;
-    if (cap == cudaStreamCaptureStatusNone) {  // a capture was prepared by prepare_grid
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem));
+    if (cap == cudaStreamCaptureStatusNone) {  // (set before a capture)
+        e = set_smem(kern, smem);
         if (e != cudaSuccess) return e;
     }
-    kern<<<grid, block, smem, s>>>(P);
+    kern<<<grid, K::threads, smem, s>>>(P);
     return cudaGetLastError();
 }
 
-// Launch the forward kernel for n_jobs jobs (P.max_inl and P.stage_cap set; P.pairs for fp32
-// storage, P.words and P.scales for 16-bit storage).
-cudaError_t launch_fwd(const FwdParams& P, int n_jobs, bool amp, int variant, cudaStream_t s,
-                       int store = psm::kStoreF32, bool kahan = false) {
+// Launch the forward kernel for n_jobs jobs (P.traces, P.store and P.max_rows set).
+cudaError_t launch_fwd(const FwdParams& P, int n_jobs, bool amp, bool narrow, cudaStream_t s,
+                       bool kahan = false, bool ordered = false) {
     if (n_jobs <= 0 || P.n_ox <= 0 || P.n_t <= 0) return cudaSuccess;
-    const size_t smem = fwd_smem(P, store);
-    if (!smem) return cudaErrorInvalidValue;
-    return with_kernel(amp, variant, store, kahan,
-                       [&](auto k) { return launch_grid(k, P, n_jobs, smem, s); });
+    auto f = [&](auto k) { return launch_grid(k, P, n_jobs, s); };
+    return ordered ? with_kernel<true>(amp, kahan, narrow, f)
+                   : with_kernel(amp, kahan, narrow, f);
 }
 
-// words[n_rows][ns] and scales[n_rows] from the fp32 rows (quantize_kernel, one warp a row).
+// 16-bit samples [n_rows][ns] and scales[n_rows] from the fp32 rows (quantize_kernel, one warp a
+// row).
 cudaError_t quantize(const float* src, uint32_t* words, float* scales, size_t n_rows, int ns,
                      int store, cudaStream_t s) {
     if (!n_rows) return cudaSuccess;
@@ -289,15 +228,6 @@ cudaError_t quantize(const float* src, uint32_t* words, float* scales, size_t n_
         psm::quantize_kernel<psm::kStoreBF16><<<blocks, 256, 0, s>>>(src, words, scales, n_rows, ns);
     else
         psm::quantize_kernel<psm::kStoreF16><<<blocks, 256, 0, s>>>(src, words, scales, n_rows, ns);
-    return cudaGetLastError();
-}
-
-// pairs[n_rows][ns] from the fp32 rows (pair_kernel).
-cudaError_t build_pairs(const float* src, float2* dst, size_t n_rows, int ns, cudaStream_t s) {
-    if (!n_rows) return cudaSuccess;
-    const size_t n = n_rows * static_cast<size_t>(ns);
-    const unsigned blocks = static_cast<unsigned>(std::min<size_t>((n + 255) / 256, 148 * 64));
-    psm::pair_kernel<<<blocks, 256, 0, s>>>(src, dst, n_rows, ns);
     return cudaGetLastError();
 }
 
@@ -328,14 +258,10 @@ int check_geometry(const psm_geom& g, std::string* why) {
         *why = "precision must be PSM_F32, PSM_BF16 or PSM_F16";
         return PSM_ERR_ARG;
     }
-    const int store = store_of(g.precision);
-    const int ns = trace_stride(g.n_t);
-    // inline window of any output inline <= 2 (m_il + pad_il) + 1 (+ the inline table) and one
-    // whole trace per ring stage must fit the CTA's shared memory
+    // inline window of any output inline <= 2 (m_il + pad_il) + 1
     const int64_t win = std::min<int64_t>(g.n_il, 2 * (int64_t(g.m_il) + g.pad_il) + 1);
-    if (psm::smem_layout(static_cast<int>(win), stage_cap(ns), 8).total > kMaxDynSmem ||
-        psm::smem_layout(static_cast<int>(win), stage_cap(ns, store), psm::store_bytes(store))
-                .total > kMaxDynSmem) {
+    if (!fits_staging(win, g.n_t, 8) ||
+        !fits_staging(win, g.n_t, store_of(g.precision) == psm::kStoreF32 ? 8 : 4)) {
         *why = "n_t / aperture too large for the staging ring";
         return PSM_ERR_UNSUPPORTED;
     }
@@ -440,10 +366,12 @@ struct psm_ctx {
     std::vector<Job> jobs;       // one per distinct migrated inline
     std::vector<Job> jobs_all;   // one per output row (term counting)
     std::vector<std::pair<int, int>> copies;  // (dst row, src row) duplicated output rows
-    // data: fp32 traces [n_il][n_xl][ns] as uploaded; pairs: the (d, d[t+1]-d) cube the
-    // forward kernel stages
-    DevBuf data, pairs, vrms, image, d_jobs, d_jobs_all, il_pos, t0, err, count;
-    // 16-bit storage: words [n_il][n_xl][ns] (q[t] | q[t+1] << 16) and one scale per trace
+    // data: fp32 traces [n_il][n_xl][ns] as uploaded, which the forward kernel stages
+    DevBuf data, vrms, image, d_jobs, d_jobs_all, il_pos, t0, err, count;
+    int tail_nt = 0;        // samples per trace up to which `data` is written, and the bytes of
+    size_t tail_bytes = 0;  // it whose rows' tails are known to be zero for that length
+    bool few = false;       // narrow tiles by default (few_tiles)
+    // 16-bit storage: samples [n_il][n_xl][ns] and one scale per trace
     DevBuf words, scales;
     // adjoint: rows of each job (fold of duplicated output rows), image upload, job images
     std::vector<int> fold_map, fold_off;
@@ -512,8 +440,8 @@ cudaError_t copy_rows(psm_ctx* c, float* img, cudaStream_t s) {
 
 FwdParams volume_params(psm_ctx* c) {
     FwdParams P{};
-    P.pairs = c->pairs.as<float2>();
-    P.words = c->words.as<uint32_t>();
+    P.traces = c->store == psm::kStoreF32 ? c->data.p : c->words.p;
+    P.store = c->store;
     P.scales = c->scales.as<float>();
     P.vrms = c->vrms.as<float>();
     P.image = c->image.as<float>();
@@ -532,9 +460,14 @@ FwdParams volume_params(psm_ctx* c) {
     P.n_ox = c->g.n_ox;
     P.xoff = -c->g.pad_xl;
     P.max_inl = max_inline_window(c->jobs_all);
-    P.stage_cap = stage_cap(c->ns, c->store);
+    P.max_rows = max_list_rows(c->jobs_all);
     fill_consts(P, c->g.dt, c->g.d_il, c->g.d_xl, c->g.tan2_theta);
     return P;
+}
+
+// Whether the ctx's forward launches use narrow tiles.
+bool ctx_narrow(const psm_ctx* c) {
+    return narrow_tiles(c->variant, c->store, c->g.compensated != 0, c->few);
 }
 
 // Host memory the CUDA driver copies through its own staging (not pinned or registered).
@@ -674,7 +607,6 @@ int psm_destroy(psm_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->data.release();
-    c->pairs.release();
     c->words.release();
     c->scales.release();
     c->vrms.release();
@@ -735,12 +667,20 @@ int psm_set_geometry(psm_ctx* c, const psm_geom* g, const int32_t* out_center) {
     c->jobs.swap(jobs);
     c->jobs_all.swap(jobs_all);
     c->copies.swap(copies);
+    c->few = few_tiles(static_cast<int64_t>(c->jobs.size()), g->n_ox, g->n_t);
     const size_t n_tr = static_cast<size_t>(g->n_il) * g->n_xl;
-    PSM_CUDA_TRY(c->st, c->data.ensure(n_tr * ns * sizeof(float)));
-    PSM_CUDA_TRY(c->st, cudaMemsetAsync(c->data.p, 0, n_tr * ns * sizeof(float), c->stream));
-    PSM_CUDA_TRY(c->st, c->pairs.ensure(n_tr * ns * sizeof(float2)));
+    const size_t cube = n_tr * ns * sizeof(float);
+    if (cube > c->data.bytes) c->tail_bytes = 0;  // reallocated below
+    PSM_CUDA_TRY(c->st, c->data.ensure(cube));
+    if (c->tail_nt != g->n_t || cube > c->tail_bytes) {
+        // the rows' tails stay zero from here on: every writer fills n_t samples of a row
+        c->tail_bytes = 0;
+        PSM_CUDA_TRY(c->st, cudaMemsetAsync(c->data.p, 0, cube, c->stream));
+        c->tail_nt = g->n_t;
+        c->tail_bytes = cube;
+    }
     if (store != psm::kStoreF32) {
-        PSM_CUDA_TRY(c->st, c->words.ensure(n_tr * ns * sizeof(uint32_t)));
+        PSM_CUDA_TRY(c->st, c->words.ensure(n_tr * ns * sizeof(uint16_t)));
         PSM_CUDA_TRY(c->st, c->scales.ensure(n_tr * sizeof(float)));
     }
     PSM_CUDA_TRY(c->st, c->vrms.ensure(n_tr * g->n_t * sizeof(float)));
@@ -801,10 +741,7 @@ int psm_set_traces(psm_ctx* c, const float* data) {
     const size_t n_tr = static_cast<size_t>(c->g.n_il) * c->g.n_xl;
     PSM_CUDA_TRY(c->st, upload_rows(c->staging, c->data.p, c->ns * sizeof(float), data,
                                     c->g.n_t * sizeof(float), n_tr, c->stream));
-    if (c->store == psm::kStoreF32)
-        PSM_CUDA_TRY(c->st, build_pairs(c->data.as<float>(), c->pairs.as<float2>(), n_tr, c->ns,
-                                        c->stream));
-    else
+    if (c->store != psm::kStoreF32)
         PSM_CUDA_TRY(c->st, quantize(c->data.as<float>(), c->words.as<uint32_t>(),
                                      c->scales.as<float>(), n_tr, c->ns, c->store, c->stream));
     PSM_CUDA_TRY(c->st, cudaStreamSynchronize(c->stream));
@@ -868,10 +805,7 @@ int psm_set_traces_segy(psm_ctx* c, const void* records, int64_t n_records, int3
             format, c->seg_pos.as<int32_t>() + r0, c->data.as<float>());
         PSM_CUDA_TRY(c->st, cudaGetLastError());
     }
-    if (c->store == psm::kStoreF32)
-        PSM_CUDA_TRY(c->st, build_pairs(c->data.as<float>(), c->pairs.as<float2>(),
-                                        static_cast<size_t>(n_tr), c->ns, s));
-    else
+    if (c->store != psm::kStoreF32)
         PSM_CUDA_TRY(c->st, quantize(c->data.as<float>(), c->words.as<uint32_t>(),
                                      c->scales.as<float>(), static_cast<size_t>(n_tr), c->ns,
                                      c->store, s));
@@ -1036,7 +970,7 @@ int psm_forward_async(psm_ctx* c) {
     PSM_CUDA_TRY(c->st, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     FwdParams P = volume_params(c);
     PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                   c->g.amp_correction != 0, c->variant, c->stream, c->store,
+                                   c->g.amp_correction != 0, ctx_narrow(c), c->stream,
                                    c->g.compensated != 0));
     // padded output inlines repeat the migrated edge inline (main.cpp:268-285)
     PSM_CUDA_TRY(c->st, copy_rows(c, c->image.as<float>(), c->stream));
@@ -1066,9 +1000,9 @@ int psm_autotune(psm_ctx* c, float* ms, int* best) {
     int pick = kDefaultVariant;
     float pick_ms = 3.0e38f;
     int rc = PSM_OK;
-    for (int v = 1; v < PSM_FWD_N_VARIANTS && rc == PSM_OK; ++v) {
-        if (effective_variant(v, c->store, c->g.compensated != 0) != v) continue;  // same kernel
-        c->variant = v;
+    // each kernel is timed once, and every variant id that runs it gets its time
+    for (int cand : {static_cast<int>(kDefaultVariant), static_cast<int>(PSM_FWD_PAIRS)}) {
+        c->variant = cand;
         float t = 0.0f;
         if ((rc = psm_forward_async(c)) != PSM_OK) break;  // warm (first launch, attribute)
         cudaEventRecord(e0, c->stream);
@@ -1076,10 +1010,14 @@ int psm_autotune(psm_ctx* c, float* ms, int* best) {
         cudaEventRecord(e1, c->stream);
         if ((rc = psm_synchronize(c)) != PSM_OK) break;
         cudaEventElapsedTime(&t, e0, e1);
-        if (ms) ms[v] = t;
+        const bool narrow = ctx_narrow(c), kahan = c->g.compensated != 0;
+        for (int v = 1; ms && v < PSM_FWD_N_VARIANTS; ++v)
+            if (effective_variant(v, c->store, kahan) == v &&
+                narrow_tiles(v, c->store, kahan, false) == narrow)
+                ms[v] = t;
         if (t < pick_ms) {
             pick_ms = t;
-            pick = v;
+            pick = cand;
         }
     }
     cudaEventDestroy(e0);
@@ -1133,8 +1071,8 @@ int forward_waves(psm_ctx* c, const float* traces, const float* vrms, float* ima
     cudaStream_t s = c->stream;
     for (cudaStream_t* t : {&c->copy_stream, &c->d2h_stream, &c->aux_stream})
         if (!*t) PSM_CUDA_TRY(c->st, cudaStreamCreateWithFlags(t, cudaStreamNonBlocking));
-    // Inputs go up in blocks of consecutive inlines: trace block b (then its pair cube or 16-bit
-    // words, built on the copy stream), and Vrms block v once the trace blocks that the output
+    // Inputs go up in blocks of consecutive inlines: trace block b (then its 16-bit samples, made
+    // on the copy stream), and Vrms block v once the trace blocks that the output
     // inlines of block v read are up (an output inline needs its whole buffer, which reaches
     // about m_il + pad_il inlines ahead, but only its own Vrms row).  A job runs in the wave of
     // the first upload after which its buffer and Vrms row are resident.  Waves alternate
@@ -1239,13 +1177,9 @@ int forward_waves(psm_ctx* c, const float* traces, const float* vrms, float* ima
             PSM_CUDA_TRY(c->st, upload_rows(c->staging, c->data.as<float>() + r0 * c->ns,
                                             c->ns * sizeof(float), traces + lo * per_il,
                                             g.n_t * sizeof(float), rows, cs));
-            if (c->store == psm::kStoreF32)
-                PSM_CUDA_TRY(c->st, build_pairs(c->data.as<float>() + r0 * c->ns,
-                                                c->pairs.as<float2>() + r0 * c->ns, rows, c->ns,
-                                                cs));
-            else
+            if (c->store != psm::kStoreF32)
                 PSM_CUDA_TRY(c->st, quantize(c->data.as<float>() + r0 * c->ns,
-                                             c->words.as<uint32_t>() + r0 * c->ns,
+                                             c->words.as<uint32_t>() + r0 * (c->ns / 2),
                                              c->scales.as<float>() + r0, rows, c->ns, c->store,
                                              cs));
         } else {
@@ -1260,7 +1194,7 @@ int forward_waves(psm_ctx* c, const float* traces, const float* vrms, float* ima
             FwdParams Q = P;
             Q.jobs = c->d_jobs_waves.as<Job>() + chunks[k].first;
             PSM_CUDA_TRY(c->st, launch_fwd(Q, chunks[k].second, g.amp_correction != 0,
-                                           c->variant, ks, c->store, g.compensated != 0));
+                                           ctx_narrow(c), ks, g.compensated != 0));
             std::vector<int> out_rows;
             for (int t = 0; t < chunks[k].second; ++t) {
                 const int r = order[chunks[k].first + t].row;
@@ -1419,17 +1353,16 @@ int adjoint_dev(psm_ctx* c, const float* d_rows, float* d_out) {
     return PSM_OK;
 }
 
-// M: data [n_il*n_xl][ns] (device, zero tail) -> image rows (device).  Rebuilds the pair
-// cube from d_vec.
-int forward_dev(psm_ctx* c, const float* d_vec, float* d_img) {
-    const size_t n_tr = static_cast<size_t>(c->g.n_il) * c->g.n_xl;
-    PSM_CUDA_TRY(c->st, build_pairs(d_vec, c->pairs.as<float2>(), n_tr, c->ns, c->stream));
+// M: data [n_il*n_xl][ns] (device, zero tail) -> image rows (device); ordered: terms added in
+// trace order (the solver's operator).
+int forward_dev(psm_ctx* c, const float* d_vec, float* d_img, bool ordered) {
     FwdParams P = volume_params(c);
+    P.traces = d_vec;
+    P.store = psm::kStoreF32;  // the operator pair of CG is the fp32 one
     P.image = d_img;
-    P.stage_cap = stage_cap(c->ns);  // the operator pair of CG is the fp32 one
     PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                   c->g.amp_correction != 0, c->variant, c->stream,
-                                   psm::kStoreF32, c->g.compensated != 0));
+                                   c->g.amp_correction != 0, ctx_narrow(c), c->stream,
+                                   c->g.compensated != 0, ordered));
     PSM_CUDA_TRY(c->st, copy_rows(c, d_img, c->stream));
     return PSM_OK;
 }
@@ -1491,7 +1424,7 @@ int psm_forward_device(psm_ctx* c, const float* d_data, float* d_image) {
     PSM_CUDA_TRY(c->st, cudaMemcpy2DAsync(c->data.p, c->ns * sizeof(float), d_data,
                                           c->g.n_t * sizeof(float), c->g.n_t * sizeof(float),
                                           n_tr, cudaMemcpyDeviceToDevice, c->stream));
-    const int r = forward_dev(c, c->data.as<float>(), d_image);
+    const int r = forward_dev(c, c->data.as<float>(), d_image, false);
     if (r) return r;
     c->have_traces = c->traces_readable = true;
     return PSM_OK;
@@ -1541,7 +1474,7 @@ int psm_lsm_cg(psm_ctx* c, const float* data, float* image, int iters, double* r
     int rc;
     // CGLS: r = d - M^T m, s = M r, p = s, gamma = <s, s>
     if ((rc = dot_dev(c, r, r, nd, hist))) return rc;
-    if ((rc = forward_dev(c, r, sv))) return rc;
+    if ((rc = forward_dev(c, r, sv, true))) return rc;
     PSM_CUDA_TRY(c->st, cudaMemcpyAsync(p, sv, nm * sizeof(float), cudaMemcpyDeviceToDevice, s));
     if ((rc = dot_dev(c, sv, sv, nm, sc + 0))) return rc;
     for (int k = 0; k < iters; ++k) {
@@ -1550,7 +1483,7 @@ int psm_lsm_cg(psm_ctx* c, const float* data, float* image, int iters, double* r
         psm::cg_alpha_kernel<<<1, 1, 0, s>>>(sc);                     // alpha = gamma / delta
         psm::cg_update_kernel<<<grid_for(nm + nd), 256, 0, s>>>(m, p, nm, r, q, nd, sc);
         if ((rc = dot_dev(c, r, r, nd, hist + k + 1))) return rc;     // ||r||^2
-        if ((rc = forward_dev(c, r, sv))) return rc;                  // s = M r
+        if ((rc = forward_dev(c, r, sv, true))) return rc;                  // s = M r
         if ((rc = dot_dev(c, sv, sv, nm, sc + 2))) return rc;         // gamma_new
         psm::cg_beta_kernel<<<1, 1, 0, s>>>(sc);                      // beta, gamma
         psm::cg_direction_kernel<<<grid_for(nm), 256, 0, s>>>(p, sv, nm, sc);  // p = s + beta p
@@ -1647,8 +1580,8 @@ extern "C" {
 int64_t psm_slab_bytes(const psm_geom* g, int32_t n_in, int32_t n_out) {
     if (!g || n_in < 0 || n_out < 0) return -1;
     const int64_t ns = trace_stride(g->n_t);
-    const int64_t stage = store_of(g->precision) == psm::kStoreF32 ? 8 : 4;
-    const int64_t per_trace = ns * (4 + 8) + (stage == 4 ? ns * 4 + 4 : 0) + 4LL * g->n_t;
+    const bool half = store_of(g->precision) != psm::kStoreF32;
+    const int64_t per_trace = ns * 4 + (half ? ns * 2 + 4 : 0) + 4LL * g->n_t;
     return int64_t(n_in) * g->n_xl * per_trace + int64_t(n_out) * g->n_ox * g->n_t * 4 +
            (int64_t(n_out) + n_in) * 64 + 4LL * g->n_t;
 }
@@ -1738,7 +1671,7 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
     const int ns = trace_stride(g->n_t);
     // Consecutive slabs' input inlines overlap (each output inline reads about m_il + pad_il
     // inlines either side), so the device window rolls: the inlines the next slab shares with
-    // this one stay on the device (pair cube or 16-bit words, and Vrms), moved to the front of
+    // this one stay on the device (fp32 or 16-bit traces, and Vrms), moved to the front of
     // their buffers, and only the new inlines are uploaded and prepared.  The new inlines of
     // slab k + 1 go up into a staging area while slab k migrates, and slab k's image returns
     // to the host while slab k + 1 migrates (two image buffers in turn), so the copies hide
@@ -1760,6 +1693,10 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
             keep[k] = std::min(slabs[k - 1].i1, sl.i1) - sl.i0;
         if (k > 0 && keep[k] > 0) max_fresh = std::max(max_fresh, (sl.i1 - sl.i0) - keep[k]);
     }
+    std::vector<Job> all, all_rows;
+    std::vector<std::pair<int, int>> reps;
+    plan_jobs(*g, out_center, all, all_rows, reps);
+    const bool few = few_tiles(static_cast<int64_t>(all.size()), g->n_ox, g->n_t);
     // size the device buffers for the widest slab once, so that none regrows
     if (n > 1 && (rc = psm_set_geometry(c, &loc[wide], lcs[wide].data()))) return rc;
     for (cudaStream_t* t : {&c->copy_stream, &c->d2h_stream})
@@ -1800,12 +1737,13 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
         const psm_slab& sl = slabs[k];
         // a buffer that set_geometry had to grow was reallocated (its size changed), and
         // its contents are gone
-        const DevBuf* bufs[4] = {&c->pairs, &c->words, &c->scales, &c->vrms};
+        const DevBuf* bufs[4] = {&c->data, &c->words, &c->scales, &c->vrms};
         size_t sizes[4];
         for (int i = 0; i < 4; ++i) sizes[i] = bufs[i]->bytes;
         const bool had = k > 0 && c->have_traces && c->have_vrms;
         // (waits for slab k - 1's kernel: psm_set_geometry synchronises the stream)
         if ((rc = psm_set_geometry(c, &loc[k], lcs[k].data()))) return rc;
+        c->few = few;  // the tiles of the whole problem: slab images are its rows bit for bit
         bool same_bufs = true;
         for (int i = 0; i < 4; ++i)
             if ((i == 0 || i == 3 || c->store != psm::kStoreF32) && bufs[i]->bytes != sizes[i])
@@ -1837,9 +1775,9 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
                 return cudaSuccess;
             };
             if (c->store == psm::kStoreF32) {
-                PSM_CUDA_TRY(c->st, move(c->pairs.p, per_il_tr * ns * sizeof(float2)));
+                PSM_CUDA_TRY(c->st, move(c->data.p, per_il_tr * ns * sizeof(float)));
             } else {
-                PSM_CUDA_TRY(c->st, move(c->words.p, per_il_tr * ns * sizeof(uint32_t)));
+                PSM_CUDA_TRY(c->st, move(c->words.p, per_il_tr * ns * sizeof(uint16_t)));
                 PSM_CUDA_TRY(c->st, move(c->scales.p, per_il_tr * sizeof(float)));
             }
             PSM_CUDA_TRY(c->st, move(c->vrms.p, trace * sizeof(float)));
@@ -1849,12 +1787,12 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
                 const size_t rows = static_cast<size_t>(fresh) * per_il_tr;
                 PSM_CUDA_TRY(c->st, cudaStreamWaitEvent(c->stream, c->ev_staged, 0));
                 if (c->store == psm::kStoreF32)
-                    PSM_CUDA_TRY(c->st, build_pairs(c->str_tr.as<float>(),
-                                                    c->pairs.as<float2>() + r0 * ns, rows, ns,
-                                                    c->stream));
+                    PSM_CUDA_TRY(c->st, cudaMemcpyAsync(c->data.as<float>() + r0 * ns,
+                                                        c->str_tr.p, rows * ns * sizeof(float),
+                                                        cudaMemcpyDeviceToDevice, c->stream));
                 else
                     PSM_CUDA_TRY(c->st, quantize(c->str_tr.as<float>(),
-                                                 c->words.as<uint32_t>() + r0 * ns,
+                                                 c->words.as<uint32_t>() + r0 * (ns / 2),
                                                  c->scales.as<float>() + r0, rows, ns, c->store,
                                                  c->stream));
                 PSM_CUDA_TRY(c->st, cudaMemcpyAsync(c->vrms.as<float>() + kp * trace,
@@ -1862,7 +1800,7 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
                                                     cudaMemcpyDeviceToDevice, c->stream));
             }
             c->have_traces = c->have_vrms = true;
-            c->traces_readable = false;  // the raw cube rows were not moved
+            c->traces_readable = false;  // (16-bit storage: the fp32 rows were not moved)
         }
         if (!direct[k]) {  // migrate slab k into image buffer k % 2
             staged = false;
@@ -1872,8 +1810,8 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
             FwdParams P = volume_params(c);
             P.image = img;
             PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                           c->g.amp_correction != 0, c->variant, c->stream,
-                                           c->store, c->g.compensated != 0));
+                                           c->g.amp_correction != 0, ctx_narrow(c), c->stream,
+                                           c->g.compensated != 0));
             PSM_CUDA_TRY(c->st, copy_rows(c, img, c->stream));  // padded inlines
             PSM_CUDA_TRY(c->st, cudaEventRecord(c->ev_done[k & 1], c->stream));
         }
@@ -1907,7 +1845,7 @@ namespace {
 struct BatchCube {
     const float* host = nullptr;
     int n_il = 0, n_xl = 0, n_t = 0, ns = 0;
-    DevBuf data, pairs, words, scales;
+    DevBuf data, words, scales;
 };
 
 struct BatchProblem {
@@ -1929,13 +1867,13 @@ struct psm_batch {
     bool amp = true, kahan = false;
     int variant = PSM_FWD_DEFAULT;
     int mode = PSM_BATCH_PERSISTENT;
-    int max_inl = 1, stage_cap = 0;
-    int max_ns = 0;  // longest trace stride over the problems
+    int max_rows = 1;
+    bool few = true;  // every problem takes narrow tiles by itself (few_tiles)
     int grid = 1;  // persistent CTAs
     int order = PSM_ORDER_DEPTH_FIRST;
-    // tile lists [time tile 128 / 256 / 512 samples (4 / 8 / 16 blocks a lane)][order]
-    int n_items[6] = {0, 0, 0, 0, 0, 0};
-    DevBuf items[6];
+    // tile lists [wide / narrow tiles][order]
+    int n_items[4] = {0, 0, 0, 0};
+    DevBuf items[4];
     std::unique_ptr<psm::BatchParams> params;  // every problem's FwdParams (kernel argument)
     DevBuf counter, il_pos;
     cudaGraphExec_t exec = nullptr;
@@ -1948,92 +1886,69 @@ struct psm_batch {
 
 namespace {
 
-// The tile list of a kernel whose time tile is 32 J samples, in the given order.
-constexpr int item_list(int J, int order) { return 2 * (J == 4 ? 0 : (J == 8 ? 1 : 2)) + order; }
-static_assert(item_list(4, 1) == 1 && item_list(8, 0) == 2 && item_list(16, 1) == 5,
-              "tile list index");
-
-// Shared-memory attribute and persistent grid (resident CTAs on every SM) of the batch
-// kernel K; done before a stream capture, so the graph holds only the launch.
-// Stage capacity of the persistent kernel K: the batch's (48 KB stages, or one whole trace),
-// or for a kernel built for 3 CTAs per SM 32 KB stages, so that three CTAs fit an SM.
+// The tile list of kernel K in the given order.
 template <class K>
-int persistent_stage_cap(const psm_batch& b) {
-    if constexpr (K::MINB > 2) return std::max(stage_cap_for(K::MINB, K::STORE), b.max_ns);
-    return b.stage_cap;
+constexpr int item_list(int order) {
+    return 2 * (K::NX == kNarrowNX) + order;
 }
 
 template <class K>
+size_t batch_smem(const psm_batch& b) {
+    return K::Layout::total(b.store, b.max_rows);
+}
+template <class K>
+auto persistent_kernel() {
+    return psm::fwd_batch_kernel<K::AMP, K::KAHAN, K::NX, K::CAP, K::MINB>;
+}
+template <class K>
+auto items_kernel() {
+    return psm::fwd_items_kernel<K::AMP, K::KAHAN, K::NX, K::CAP, K::MINB>;
+}
+
+// Shared-memory attribute and persistent grid (resident CTAs on every SM) of the batch
+// kernel K; done before a stream capture, so the graph holds only the launch.
+template <class K>
 cudaError_t prepare_persistent(K, psm_batch& b) {
-    auto* kern = psm::fwd_batch_kernel<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN,
-                                       K::PAIRS, K::MINB>;
-    const size_t smem =
-        psm::smem_layout(b.max_inl, persistent_stage_cap<K>(b), psm::store_bytes(K::STORE))
-            .total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    auto* kern = persistent_kernel<K>();
+    const size_t smem = batch_smem<K>(b);
+    cudaError_t e = set_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0, n_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * (psm::kTX + 1), smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, K::threads, smem);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b.ctx->device);
     if (e != cudaSuccess) return e;
-    const int w = item_list(K::J, b.order);
-    b.grid = std::max(1, std::min(b.n_items[w], n_sm * std::max(per_sm, 1)));
+    b.grid = std::max(1, std::min(b.n_items[item_list<K>(b.order)], n_sm * std::max(per_sm, 1)));
     return cudaSuccess;
 }
 
 template <class K>
 cudaError_t launch_persistent(K, const psm_batch& b, cudaStream_t s) {
-    auto* kern = psm::fwd_batch_kernel<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN,
-                                       K::PAIRS, K::MINB>;
-    const int cap = persistent_stage_cap<K>(b);
-    const size_t smem = psm::smem_layout(b.max_inl, cap, psm::store_bytes(K::STORE)).total;
-    const int w = item_list(K::J, b.order);
-    const psm::BatchParams* params = b.params.get();
-    std::unique_ptr<psm::BatchParams> small;
-    if constexpr (K::MINB > 2) {  // every problem stages into the smaller stages
-        small = std::make_unique<psm::BatchParams>(*b.params);
-        for (size_t i = 0; i < b.probs.size(); ++i) small->p[i].stage_cap = cap;
-        params = small.get();
-    }
-    kern<<<b.grid, 32 * (psm::kTX + 1), smem, s>>>(
-        *params, b.items[w].as<psm::BatchItem>(), b.n_items[w], b.counter.as<int>(),
-        b.ctx->err.as<int>(), b.max_inl, cap);
+    const int w = item_list<K>(b.order);
+    persistent_kernel<K>()<<<b.grid, K::threads, batch_smem<K>(b), s>>>(
+        *b.params, b.items[w].as<psm::BatchItem>(), b.n_items[w], b.counter.as<int>(),
+        b.ctx->err.as<int>());
     return cudaGetLastError();
 }
 
-// The one-grid kernel K (a CTA per tile of the list): its shared-memory attribute, set before
-// a stream capture.
-template <class K>
-cudaError_t prepare_items(K, const psm_batch& b) {
-    auto* kern = psm::fwd_items_kernel<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN,
-                                       K::PAIRS, K::MINB>;
-    const size_t smem =
-        psm::smem_layout(b.max_inl, persistent_stage_cap<K>(b), psm::store_bytes(K::STORE))
-            .total;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem));
-}
-
+// The one-grid kernel K (a CTA per tile of the list).
 template <class K>
 cudaError_t launch_items(K, const psm_batch& b, cudaStream_t s) {
-    auto* kern = psm::fwd_items_kernel<K::AMP, K::PACKED, K::GB, K::J, K::STORE, K::KAHAN,
-                                       K::PAIRS, K::MINB>;
-    const int cap = persistent_stage_cap<K>(b);
-    const size_t smem = psm::smem_layout(b.max_inl, cap, psm::store_bytes(K::STORE)).total;
-    const int w = item_list(K::J, b.order);
+    const int w = item_list<K>(b.order);
     if (b.n_items[w] <= 0) return cudaSuccess;
-    const psm::BatchParams* params = b.params.get();
-    std::unique_ptr<psm::BatchParams> small;
-    if constexpr (K::MINB > 2) {  // every problem stages into the smaller stages
-        small = std::make_unique<psm::BatchParams>(*b.params);
-        for (size_t i = 0; i < b.probs.size(); ++i) small->p[i].stage_cap = cap;
-        params = small.get();
-    }
-    kern<<<b.n_items[w], 32 * (psm::kTX + 1), smem, s>>>(
-        *params, b.items[w].as<psm::BatchItem>(), b.max_inl, cap);
+    items_kernel<K>()<<<b.n_items[w], K::threads, batch_smem<K>(b), s>>>(
+        *b.params, b.items[w].as<psm::BatchItem>());
     return cudaGetLastError();
+}
+
+// Tiles of a launch of every problem, and of one problem's own launch.
+bool batch_narrow(const psm_batch& b) {
+    return narrow_tiles(b.variant, b.store, b.kahan, b.few);
+}
+bool problem_narrow(const psm_batch& b, const BatchProblem& p) {
+    return narrow_tiles(b.variant, b.store, b.kahan,
+                        few_tiles(static_cast<int64_t>(p.jobs.size()), p.src.geom.n_ox,
+                                  p.src.geom.n_t));
 }
 
 // Repeated output rows of every problem (padded output inlines, main.cpp:268-285).
@@ -2052,57 +1967,58 @@ cudaError_t batch_copies(const psm_batch& b, cudaStream_t s) {
 
 // The work of one batched run, enqueued on s (persistent: counter and error word reset, one
 // launch, row copies).
-cudaError_t batch_enqueue(psm_batch& b, int variant, cudaStream_t s) {
+cudaError_t batch_enqueue(psm_batch& b, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b.ctx->err.p, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
     if (b.mode == PSM_BATCH_ONE_GRID) {
-        e = with_kernel(b.amp, variant, b.store, b.kahan,
+        e = with_kernel(b.amp, b.kahan, batch_narrow(b),
                         [&](auto k) { return launch_items(k, b, s); });
         if (e != cudaSuccess) return e;
     } else if (b.mode == PSM_BATCH_PER_PROBLEM) {
         for (const BatchProblem& p : b.probs) {
-            e = launch_fwd(p.P, static_cast<int>(p.jobs.size()), b.amp, variant, s, b.store,
+            e = launch_fwd(p.P, static_cast<int>(p.jobs.size()), b.amp, problem_narrow(b, p), s,
                            b.kahan);
             if (e != cudaSuccess) return e;
         }
     } else {
         e = cudaMemsetAsync(b.counter.p, 0, sizeof(int), s);
         if (e != cudaSuccess) return e;
-        e = with_kernel(b.amp, variant, b.store, b.kahan,
+        e = with_kernel(b.amp, b.kahan, batch_narrow(b),
                         [&](auto k) { return launch_persistent(k, b, s); });
         if (e != cudaSuccess) return e;
     }
     return batch_copies(b, s);
 }
 
-// Capture the run (either mode) into a CUDA graph once per variant, order and mode, then
+// Capture the run (any mode) into a CUDA graph once per variant, order and mode, then
 // replay it.
 int batch_launch(psm_batch* b) {
     psm_ctx* c = b->ctx;
-    const int v = effective_variant(b->variant, b->store, b->kahan);
-    const int key = (v * 2 + b->order) * 3 + b->mode;
+    const int key = (b->variant * 2 + b->order) * 3 + b->mode;
     if (!b->exec || b->exec_key != key) {
         if (b->exec) {
             cudaGraphExecDestroy(b->exec);
             b->exec = nullptr;
         }
+        // the kernels' shared-memory attributes are set outside the capture
         if (b->mode == PSM_BATCH_ONE_GRID)
-            PSM_CUDA_TRY(c->st, with_kernel(b->amp, v, b->store, b->kahan, [&](auto k) {
-                             return prepare_items(k, *b);
+            PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
+                             using K = decltype(k);
+                             return set_smem(items_kernel<K>(), batch_smem<K>(*b));
                          }));
         else if (b->mode == PSM_BATCH_PERSISTENT)
-            PSM_CUDA_TRY(c->st, with_kernel(b->amp, v, b->store, b->kahan, [&](auto k) {
+            PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
                              return prepare_persistent(k, *b);
                          }));
-        else {  // grid launches: the shared-memory attribute is set outside the capture
-            size_t smem = 0;
-            for (const BatchProblem& p : b->probs) smem = std::max(smem, fwd_smem(p.P, b->store));
-            PSM_CUDA_TRY(c->st, with_kernel(b->amp, v, b->store, b->kahan,
-                                            [&](auto k) { return prepare_grid(k, smem); }));
-        }
+        else
+            for (bool narrow : {false, true})
+                PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, narrow, [&](auto k) {
+                                 using K = decltype(k);
+                                 return set_smem(grid_kernel<K>(), batch_smem<K>(*b));
+                             }));
         cudaGraph_t graph = nullptr;
         PSM_CUDA_TRY(c->st, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        const cudaError_t e = batch_enqueue(*b, v, c->stream);
+        const cudaError_t e = batch_enqueue(*b, c->stream);
         const cudaError_t e2 = cudaStreamEndCapture(c->stream, &graph);
         PSM_CUDA_TRY(c->st, e);
         PSM_CUDA_TRY(c->st, e2);
@@ -2123,10 +2039,7 @@ int batch_upload(psm_batch* b) {
         const size_t n_tr = static_cast<size_t>(q.n_il) * q.n_xl;
         PSM_CUDA_TRY(c->st, upload_rows(c->staging, q.data.p, q.ns * sizeof(float), q.host,
                                         q.n_t * sizeof(float), n_tr, s));
-        if (b->store == psm::kStoreF32)
-            PSM_CUDA_TRY(c->st, build_pairs(q.data.as<float>(), q.pairs.as<float2>(), n_tr,
-                                            q.ns, s));
-        else
+        if (b->store != psm::kStoreF32)
             PSM_CUDA_TRY(c->st, quantize(q.data.as<float>(), q.words.as<uint32_t>(),
                                          q.scales.as<float>(), n_tr, q.ns, b->store, s));
     }
@@ -2165,7 +2078,7 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
     b->store = store_of(g0.precision);
     b->amp = g0.amp_correction != 0;
     b->kahan = g0.compensated != 0;
-    int max_il = 1;
+    int max_il = 1, max_inl = 1, max_nt = 1;
     for (int i = 0; i < n; ++i) {
         const psm_problem& src = problems[i];
         const psm_geom& g = src.geom;
@@ -2205,12 +2118,12 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
         }
         p.cube = cube;
         max_il = std::max(max_il, g.n_il);
-        b->max_inl = std::max(b->max_inl, max_inline_window(p.jobs_all));
-        b->stage_cap = std::max(b->stage_cap, stage_cap(trace_stride(g.n_t), b->store));
-        b->max_ns = std::max(b->max_ns, trace_stride(g.n_t));
+        max_inl = std::max(max_inl, max_inline_window(p.jobs_all));
+        max_nt = std::max(max_nt, g.n_t);
+        b->max_rows = std::max(b->max_rows, max_list_rows(p.jobs_all));
+        b->few = b->few && few_tiles(static_cast<int64_t>(p.jobs.size()), g.n_ox, g.n_t);
     }
-    if (psm::smem_layout(b->max_inl, b->stage_cap, psm::store_bytes(b->store)).total >
-        kMaxDynSmem)
+    if (!fits_staging(max_inl, max_nt, b->store == psm::kStoreF32 ? 8 : 4))
         return c->st.fail(PSM_ERR_UNSUPPORTED, "problems too large for one staging ring");
     cudaStream_t s = c->stream;
     PSM_CUDA_TRY(c->st, c->err.ensure(sizeof(int)));
@@ -2218,10 +2131,8 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
         const size_t n = static_cast<size_t>(q.n_il) * q.n_xl * q.ns;
         PSM_CUDA_TRY(c->st, q.data.ensure(n * sizeof(float)));
         PSM_CUDA_TRY(c->st, cudaMemsetAsync(q.data.p, 0, n * sizeof(float), s));
-        if (b->store == psm::kStoreF32) {
-            PSM_CUDA_TRY(c->st, q.pairs.ensure(n * sizeof(float2)));
-        } else {
-            PSM_CUDA_TRY(c->st, q.words.ensure(n * sizeof(uint32_t)));
+        if (b->store != psm::kStoreF32) {
+            PSM_CUDA_TRY(c->st, q.words.ensure(n * sizeof(uint16_t)));
             PSM_CUDA_TRY(c->st, q.scales.ensure(static_cast<size_t>(q.n_il) * q.n_xl *
                                                 sizeof(float)));
         }
@@ -2263,8 +2174,8 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
                                                 cudaMemcpyHostToDevice, s));
         }
         FwdParams& P = p.P;
-        P.pairs = q.pairs.as<float2>();
-        P.words = q.words.as<uint32_t>();
+        P.traces = b->store == psm::kStoreF32 ? q.data.p : q.words.p;
+        P.store = b->store;
         P.scales = q.scales.as<float>();
         P.vrms = p.vrms.as<float>();
         P.image = p.image.as<float>();
@@ -2283,27 +2194,27 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
         P.n_ox = g.n_ox;
         P.xoff = -g.pad_xl;
         P.max_inl = max_inline_window(p.jobs_all);
-        P.stage_cap = stage_cap(q.ns, b->store);
+        P.max_rows = b->max_rows;  // (the batch's: its kernels' shared memory is laid out once)
         fill_consts(P, g.dt, g.d_il, g.d_xl, g.tan2_theta);
         if (vk != PSM_VRMS_CUBE) P.vs_x = P.vs_row = 0;  // one Vrms trace for every point
         b->params->p[i] = P;
     }
-    // tile lists, for 128-, 256- and 512-sample time tiles, in two orders:
+    // tile lists, for wide and narrow tiles, in two orders:
     //  * depth first: deepest time tiles first (the aperture, and so the work, grows with
     //    t0), then output inline, crossline tile and problem, so panels over one cube take
     //    the same tile one after another and the long tiles start early;
     //  * problem after problem, each in the grid kernel's order (crossline tile fastest,
     //    then output inline, then time tile, deepest first).
     PSM_CUDA_TRY(c->st, b->counter.ensure(sizeof(int)));
-    for (int w = 0; w < 6; ++w) {
-        const int TT = 32 * (4 << (w / 2));
+    for (int w = 0; w < 4; ++w) {
+        const int TT = psm::kTileT, NX = w < 2 ? kWideNX : kNarrowNX;
         std::vector<psm::BatchItem> items;
         for (int i = 0; i < n; ++i) {
             const BatchProblem& p = b->probs[i];
             const psm_geom& g = p.src.geom;
             for (int T0 = (g.n_t - 1) / TT * TT; T0 >= 0; T0 -= TT)
                 for (int j = 0; j < static_cast<int>(p.jobs.size()); ++j)
-                    for (int x0 = 0; x0 < g.n_ox; x0 += psm::kTX) items.push_back({i, j, x0, T0});
+                    for (int x0 = 0; x0 < g.n_ox; x0 += NX) items.push_back({i, j, x0, T0});
         }
         if ((w & 1) == PSM_ORDER_DEPTH_FIRST)
             std::stable_sort(items.begin(), items.end(),
@@ -2413,9 +2324,9 @@ int psm_batch_autotune(psm_batch* b, float* ms, int* best, int* best_order, int*
         b->mode = sch < 2 ? PSM_BATCH_PERSISTENT
                           : (sch == 2 ? PSM_BATCH_PER_PROBLEM : PSM_BATCH_ONE_GRID);
         b->order = sch < 2 ? sch : (sch == 2 ? PSM_ORDER_DEPTH_FIRST : sch - 3);
-        for (int v = 1; v < PSM_FWD_N_VARIANTS && rc == PSM_OK; ++v) {
-            if (effective_variant(v, b->store, b->kahan) != v) continue;  // same kernel
-            b->variant = v;
+        // each kernel is timed once, and every variant id that runs it gets its time
+        for (int cand : {static_cast<int>(kDefaultVariant), static_cast<int>(PSM_FWD_PAIRS)}) {
+            b->variant = cand;
             float t = 0.0f;
             if ((rc = psm_batch_run(b)) != PSM_OK) break;  // warm: graph capture, first launch
             cudaEventRecord(e0, c->stream);
@@ -2423,10 +2334,14 @@ int psm_batch_autotune(psm_batch* b, float* ms, int* best, int* best_order, int*
             cudaEventRecord(e1, c->stream);
             if ((rc = psm_batch_synchronize(b)) != PSM_OK) break;
             cudaEventElapsedTime(&t, e0, e1);
-            if (ms) ms[sch * PSM_FWD_N_VARIANTS + v] = t;
+            const bool narrow = batch_narrow(*b);
+            for (int v = 1; ms && v < PSM_FWD_N_VARIANTS; ++v)
+                if (effective_variant(v, b->store, b->kahan) == v &&
+                    narrow_tiles(v, b->store, b->kahan, false) == narrow)
+                    ms[sch * PSM_FWD_N_VARIANTS + v] = t;
             if (t < pick_ms) {
                 pick_ms = t;
-                pick = v;
+                pick = cand;
                 pick_order = b->order;
                 pick_mode = b->mode;
             }
@@ -2503,7 +2418,7 @@ struct InlineStaging {
     int device = -1;
     cudaStream_t stream = nullptr;
     Status st;
-    DevBuf data, pairs, vel, out, job, il_pos, t0, err;
+    DevBuf data, vel, out, job, il_pos, t0, err;
     ~InlineStaging() {
         if (stream) cudaStreamDestroy(stream);
     }
@@ -2532,8 +2447,8 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
         return PSM_ERR_ARG;
     }
     const int ns = trace_stride(static_cast<int>(n_t));
-    if (psm::smem_layout(std::max<int>(static_cast<int>(n_buf_il), 1), stage_cap(ns)).total >
-        kMaxDynSmem) {
+    if (!fits_staging(std::max<int64_t>(static_cast<int64_t>(n_buf_il), 1),
+                      static_cast<int>(n_t), 8)) {
         tl_inline_error = "n_t / buffer too large for the staging ring";
         return PSM_ERR_UNSUPPORTED;
     }
@@ -2561,7 +2476,6 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
     }
     const size_t n_tr = n_buf_il * n_buf_xl;
     PSM_INL_TRY(S->data.ensure(std::max<size_t>(n_tr, 1) * ns * sizeof(float)));
-    PSM_INL_TRY(S->pairs.ensure(std::max<size_t>(n_tr, 1) * ns * sizeof(float2)));
     PSM_INL_TRY(S->vel.ensure(std::max<size_t>(n_buf_xl, 1) * n_t * sizeof(float)));
     PSM_INL_TRY(S->out.ensure(n_out_xl * n_t * sizeof(float)));
     PSM_INL_TRY(S->job.ensure(sizeof(Job)));
@@ -2574,7 +2488,6 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
         PSM_INL_TRY(cudaMemcpy2DAsync(S->data.p, ns * sizeof(float), input_buffer,
                                       n_t * sizeof(float), n_t * sizeof(float), n_tr,
                                       cudaMemcpyHostToDevice, s));
-        PSM_INL_TRY(build_pairs(S->data.as<float>(), S->pairs.as<float2>(), n_tr, ns, s));
     }
     if (n_buf_xl)
         PSM_INL_TRY(cudaMemcpyAsync(S->vel.p, velocity_slice, n_buf_xl * n_t * sizeof(float),
@@ -2592,7 +2505,8 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
     PSM_INL_TRY(cudaMemcpyAsync(S->job.p, &j, sizeof(Job), cudaMemcpyHostToDevice, s));
     PSM_INL_TRY(cudaMemsetAsync(S->err.p, 0, sizeof(int), s));
     FwdParams P{};
-    P.pairs = S->pairs.as<float2>();
+    P.traces = S->data.p;
+    P.store = psm::kStoreF32;
     P.vrms = S->vel.as<float>();
     P.image = S->out.as<float>();
     P.jobs = S->job.as<Job>();
@@ -2607,11 +2521,11 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
     P.n_ox = static_cast<int>(n_out_xl);
     P.xoff = current_xl_start;
     P.max_inl = std::max<int>(static_cast<int>(n_buf_il), 1);
-    P.stage_cap = stage_cap(ns);
     fill_consts(P, dt, inline_bin_size, crossline_bin_size, tan_theta_sq);
     for (size_t i = 1; i < n_buf_il; ++i)  // mirrored pairs need consecutive inline positions
         if (il_pos_indices[i] != il_pos_indices[i - 1] + 1) P.pairable = 0;
-    PSM_INL_TRY(launch_fwd(P, 1, amp_correction != 0, PSM_FWD_DEFAULT, s));
+    P.max_rows = P.pairable && n_buf_il ? list_rows(cur - il_pos_indices[0], P.max_inl) : P.max_inl;
+    PSM_INL_TRY(launch_fwd(P, 1, amp_correction != 0, few_tiles(1, P.n_ox, P.n_t), s));
     PSM_INL_TRY(cudaMemcpyAsync(output_slice, S->out.p, n_out_xl * n_t * sizeof(float),
                                 cudaMemcpyDeviceToHost, s));
     int h = 0;
@@ -2696,7 +2610,7 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
         return PSM_ERR_ARG;
     if (g->n_oi > kNoallocMaxRows || g->n_il > kNoallocMaxInl || g->n_t > kNoallocMaxT)
         return PSM_ERR_UNSUPPORTED;
-    const int ns = trace_stride(g->n_t);
+    const int ns = (g->n_t + 7) & ~7;  // the caller's rows of pairs
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     NoallocTables& T = g_noalloc_tables;
@@ -2706,7 +2620,7 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
     Job* jobs = T.jobs;
     int16_t* first_row_of = T.first_row_of;
     int16_t *dup_dst = T.dup_dst, *dup_src = T.dup_src;
-    int n_jobs = 0, n_dup = 0, max_inl = 1;
+    int n_jobs = 0, n_dup = 0, max_inl = 1, max_rows = 1;
     for (int i = 0; i < g->n_il; ++i) first_row_of[i] = -1;
     for (int o = 0; o < g->n_oi; ++o) {
         const int cc = out_center ? out_center[o]
@@ -2715,6 +2629,7 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
         const int rs = std::max(0, cc - g->m_il), re = std::min(g->n_il, cc + g->m_il + 1);
         Job j{o, cc, cc, std::max(0, rs - g->pad_il), std::min(g->n_il, re + g->pad_il)};
         max_inl = std::max(max_inl, j.i1 - j.i0);
+        max_rows = std::max(max_rows, list_rows(j.pos - j.i0, j.i1 - j.i0));
         if (first_row_of[cc] < 0) {
             first_row_of[cc] = static_cast<int16_t>(o);
             jobs[n_jobs++] = j;
@@ -2733,8 +2648,8 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
     P.n_ox = g->n_ox;
     P.xoff = -g->pad_xl;
     P.max_inl = max_inl;
-    P.stage_cap = stage_cap(ns);
-    if (!fwd_smem(P)) return PSM_ERR_UNSUPPORTED;
+    P.max_rows = max_rows;
+    if (!fits_staging(max_inl, g->n_t, 8)) return PSM_ERR_UNSUPPORTED;
     fill_consts(P, g->dt, g->d_il, g->d_xl, g->tan2_theta);
 
     unsigned char* scratch = nullptr;
@@ -2756,14 +2671,15 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
                                cudaMemcpyHostToDevice, s));
     PSM_NA_TRY(cudaMemcpyAsync(scratch + kNoallocT0, t0, sizeof(float) * g->n_t,
                                cudaMemcpyHostToDevice, s));
-    P.pairs = reinterpret_cast<const float2*>(d_pairs);
+    P.traces = d_pairs;
+    P.store = psm::kStorePairs;
     P.vrms = d_vrms;
     P.image = d_image;
     P.jobs = reinterpret_cast<const Job*>(scratch + kNoallocJobs);
     P.il_pos = reinterpret_cast<const int*>(scratch + kNoallocPos);
     P.t0 = reinterpret_cast<const float*>(scratch + kNoallocT0);
     P.err = reinterpret_cast<int*>(scratch + kNoallocErr);
-    PSM_NA_TRY(launch_fwd(P, n_jobs, g->amp_correction != 0, PSM_FWD_DEFAULT, s));
+    PSM_NA_TRY(launch_fwd(P, n_jobs, g->amp_correction != 0, few_tiles(n_jobs, g->n_ox, g->n_t), s));
     const size_t row = static_cast<size_t>(g->n_ox) * g->n_t;
     for (int k = 0; k < n_dup; ++k)
         PSM_NA_TRY(cudaMemcpyAsync(d_image + dup_dst[k] * row, d_image + dup_src[k] * row,

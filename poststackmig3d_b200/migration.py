@@ -450,10 +450,9 @@ class Migrator:
                                  hist.ctypes.data), self._err)
         return img, hist
 
-    VARIANTS = {1: "scalar/g2", 2: "scalar/g4", 3: "packed/g2", 4: "packed/g4",
-                5: "packed/g4/j16", 6: "scalar/g4/j16", 7: "packed/g8", 8: "scalar/g8",
-                9: "packed/g4/o3", 10: "scalar/g4/o3", 11: "pairs/o3", 12: "pairs",
-                13: "pairs/j4/o4"}
+    # ids and the kernel each runs: tiles of 14 output crosslines (wide) or of 4 (narrow)
+    VARIANTS = {**{v: "pairs/wide" for v in range(1, 12)}, 12: "pairs/narrow",
+                13: "pairs/narrow"}
 
     def set_variant(self, variant: int) -> None:
         check(self._L.psm_set_variant(self._ctx, int(variant)), self._err)
@@ -464,8 +463,8 @@ class Migrator:
         return v.value
 
     def autotune(self):
-        """Time every forward variant once on the resident cube and keep the fastest.
-        Returns (best variant, {variant: ms})."""
+        """Time each forward kernel once on the resident cube and keep the fastest.
+        Returns (best variant, {variant: its kernel's ms})."""
         ms = np.zeros(max(self.VARIANTS) + 1, dtype=np.float32)
         best = ctypes.c_int()
         check(self._L.psm_autotune(self._ctx, ms.ctypes.data, ctypes.byref(best)), self._err)
@@ -585,7 +584,7 @@ class Batch:
         return v.value
 
     def autotune(self):
-        """Time every kernel variant on each schedule (SCHEDULES: persistent depth-first /
+        """Time each kernel on each schedule (SCHEDULES: persistent depth-first /
         problem order, per-problem launches, one grid depth-first / problem order); keep the
         fastest.  Returns (variant, order, mode, {(variant, schedule): ms})."""
         nv = max(Migrator.VARIANTS) + 1
