@@ -8,11 +8,12 @@
 // for exactly the same terms (same masks B, same travel time, same frac and q), so the pair
 // passes the dot-product test to FP32 summation noise.
 //
-// Same tile decomposition as fwd_kernel.  The producer stages no data: each ring stage is a
-// zeroed shared-memory accumulator holding one fp32 window per listed trace; consumers add
-// into it with shared-memory atomics; once a stage is released, the producer adds every
-// window into the data cube in HBM with a TMA bulk reduction (cp.reduce.async.bulk .add.f32)
-// and waits for the reduction to have read the stage before zeroing and reusing it.  As in
+// A tile is an output inline, kTX output crosslines (a consumer warp each) and kTT samples.  The
+// producer stages no data: each ring stage is a zeroed shared-memory accumulator holding one
+// fp32 window per listed trace; consumers add into it; once a stage is released, the producer
+// adds every window into the data cube in HBM with a TMA bulk reduction
+// (cp.reduce.async.bulk .add.f32) and waits for the reduction to have read the stage before
+// zeroing and reusing it.  As in
 // the forward, the traces at inlines c - d and c + d of one crossline (mirrored about the
 // output inline c) have the same r^2 to every output point, hence the same travel times,
 // fractions and weights: every term adds the same two shares to both.  They share one slot
@@ -212,37 +213,163 @@ __device__ __forceinline__ void adj_term2(unsigned char* sbase, float r2, uint32
     }
 }
 
-template <bool AMP, bool FIX>
-__device__ __forceinline__ void adj_visit(unsigned char* sbase, float r2, uint32_t base,
-                                          float smax,
-                                          const float (&gmax)[2], const float (&gmin)[2],
-                                          const float (&T2)[kJ], const float (&F4)[kJ],
-                                          const float (&BB)[kJ], const float (&MK)[kJ]) {
+template <bool AMP>
+__device__ __forceinline__ void adj_visit_fixed(unsigned char* sbase, float r2, uint32_t base,
+                                                float smax, const float (&gmax)[2],
+                                                const float (&gmin)[2], const float2 (&T2)[kJ / 2],
+                                                const float2 (&F4)[kJ / 2],
+                                                const float2 (&BB)[kJ / 2],
+                                                const float2 (&MK)[kJ / 2]) {
 #pragma unroll
-    for (int gr = 0; gr < 2; ++gr) {
-        if (r2 <= gmax[gr]) {
-            if (FIX) {  // exact integer shares: each term on its own
-                if (r2 <= gmin[gr]) {
+    for (int h = 0; h < 2; ++h) {
+        if (r2 <= gmax[h]) {  // exact integer shares: each term on its own
 #pragma unroll
-                    for (int j = 4 * gr; j < 4 * gr + 4; ++j)
-                        adj_term<AMP, false, FIX>(sbase, r2, base, smax, T2[j], F4[j], BB[j],
-                                                  MK[j]);
+            for (int p = 2 * h; p < 2 * h + 2; ++p) {
+                if (r2 <= gmin[h]) {
+                    adj_term<AMP, false, true>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
+                                               MK[p].x);
+                    adj_term<AMP, false, true>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
+                                               MK[p].y);
                 } else {
-#pragma unroll
-                    for (int j = 4 * gr; j < 4 * gr + 4; ++j)
-                        adj_term<AMP, true, FIX>(sbase, r2, base, smax, T2[j], F4[j], BB[j],
-                                                 MK[j]);
+                    adj_term<AMP, true, true>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
+                                              MK[p].x);
+                    adj_term<AMP, true, true>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
+                                              MK[p].y);
                 }
-            } else if (r2 <= gmin[gr]) {  // blocks j, j + 1 hold samples t, t + 1
+            }
+        }
+    }
+}
+
+// fp32 sums without atomics.  The warp owns the slot's window while it adds (see the consumers),
+// so a lane may load, add and store; what must not happen is that two lanes of one step hold
+// the same address.  A lane's samples t, t + 1 touch at most the addresses l, l + 1, l + 2 with
+// l = floor(s(t)), and below the couple's r^2 bound `safe` (safe_reach) l grows from lane to
+// lane and from block to block, so the lanes' addresses l + k of one k are distinct: three
+// steps, k = 0, 1, 2, with a warp barrier between them.  Two blocks of 64 samples go together
+// (two independent chains of load, add and store).  A lane whose second sample lands beyond
+// l + 1 (rounding at ds/dt0 = 1, a falling Vrms) sends its blocks through the atomics.
+// N blocks of 64 samples go together (independent chains of load, add and store).
+// floor(s) of a passing term is n_t - 1 at most (a fast s that rounds up): its share beyond the
+// record falls on the window's sample n_t, which the flush drops.
+// False when it left the blocks to the atomics.
+template <bool AMP, bool MASK, int N>
+__device__ __forceinline__ bool adj_add(unsigned char* sbase, float r2, uint32_t base,
+                                        const float2* T2, const float2* F4, const float2* BB,
+                                        const float2* MK) {
+    float* at[N];
+    float a0[N], a1[N], a2[N];
+    bool act[N], two[N], far = false;
 #pragma unroll
-                for (int j = 4 * gr; j < 4 * gr + 4; j += 2)
-                    adj_term2<AMP, false>(sbase, r2, base, smax, T2[j], F4[j], BB[j], MK[j],
-                                          T2[j + 1], F4[j + 1], BB[j + 1], MK[j + 1]);
-            } else {
+    for (int j = 0; j < N; ++j) {
+        const bool oka = !MASK || r2 <= BB[j].x, okb = !MASK || r2 <= BB[j].y;
+        const float2 t2 = fma2(F4[j], make_float2(r2, r2), T2[j]);
+        const float2 q = make_float2(rsqrtf(t2.x), rsqrtf(t2.y));
+        const float2 s = mul2(t2, q);
+        const float2 M = make_float2(8388608.0f, 8388608.0f);
+        const float2 mm = add2_rm(s, M);
+        const float2 fr = sub2(s, sub2(mm, M));
+        float2 c = AMP ? mul2(MK[j], q) : MK[j];
+        if (MASK) c = make_float2(oka ? c.x : 0.0f, okb ? c.y : 0.0f);
+        const float2 c1 = mul2(c, fr), c0 = sub2(c, c1);
+        const uint32_t la = __float_as_uint(mm.x), d = __float_as_uint(mm.y) - la;
+        at[j] = reinterpret_cast<float*>(sbase + (base + (la << 2)));
+        const bool same = d == 0u;
+        a0[j] = c0.x + (same ? c0.y : 0.0f);
+        a1[j] = c1.x + (same ? c1.y : c0.y);
+        a2[j] = c1.y;
+        act[j] = oka || okb;
+        two[j] = okb && d == 1u;
+        far = far || (okb && d > 1u);
+    }
+    if (__any_sync(0xffffffffu, far)) return false;
+    float x[N];
 #pragma unroll
-                for (int j = 4 * gr; j < 4 * gr + 4; j += 2)
-                    adj_term2<AMP, true>(sbase, r2, base, smax, T2[j], F4[j], BB[j], MK[j],
-                                         T2[j + 1], F4[j + 1], BB[j + 1], MK[j + 1]);
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (k < 2 ? act[j] : two[j]) x[j] = at[j][k];
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (k < 2 ? act[j] : two[j]) at[j][k] = x[j] + (k == 0 ? a0[j] : k == 1 ? a1[j] : a2[j]);
+        __syncwarp();
+    }
+    return true;
+}
+
+constexpr float kBeyond = 3.0e38f;  // (t / dt)^2 of a sample beyond the record: above every other
+
+// Largest r^2 up to `top` for which s(t') - s(t) >= 1.01 (so that their floors differ, rounding
+// included), t' the sample that the next lane (or block) holds: with s^2 = T2 + F4 r^2 that is
+// (T2' - T2) + r^2 (F4' - F4) >= 1.01 (s + s').  The left side less the right side falls with r^2
+// once F4' - F4 is held at 0 or below (a falling Vrms would only help), so the good r^2 form a
+// prefix; found by bisection where the far end fails.
+__device__ __forceinline__ float safe_reach(float ta, float fa, float tb, float fb, float top) {
+    const float dt = tb - ta, df = fminf(fb - fa, 0.0f);
+    auto good = [&](float r2) {
+        return fmaf(r2, df, dt) >=
+               1.01f * (sqrtf(fmaf(fa, r2, ta)) + sqrtf(fmaf(fb, r2, tb)));
+    };
+    if (good(top)) return 3.0e38f;
+    if (!good(0.0f)) return -1.0f;
+    float lo = 0.0f, hi = top;
+    for (int i = 0; i < 12; ++i) {
+        const float mid = 0.5f * (lo + hi);
+        if (good(mid))
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ void consumer_barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kTX) : "memory");
+}
+// True when every consumer thread calls it with true.
+__device__ __forceinline__ bool consumers_agree(bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"(static_cast<uint32_t>(ok)), "n"(32 * kTX)
+        : "memory");
+    return r != 0;
+}
+
+template <bool AMP>
+__device__ __forceinline__ void adj_visit(unsigned char* sbase, float r2, uint32_t base,
+                                          float smax, const float (&gmax)[2],
+                                          const float (&gmin)[2], const float (&safe)[2],
+                                          const float2 (&T2)[kJ / 2], const float2 (&F4)[kJ / 2],
+                                          const float2 (&BB)[kJ / 2],
+                                          const float2 (&MK)[kJ / 2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (r2 <= gmax[h]) {
+            const int p = 2 * h, n = p + 1;
+            bool done = false;
+            if (r2 <= safe[h]) {
+                if (r2 <= gmin[h]) {
+                    done = adj_add<AMP, false, 2>(sbase, r2, base, T2 + p, F4 + p, BB + p, MK + p);
+                } else {  // a block without a passing lane is left out
+                    const bool a = __any_sync(0xffffffffu, r2 <= fmaxf(BB[p].x, BB[p].y));
+                    const bool b = __any_sync(0xffffffffu, r2 <= fmaxf(BB[n].x, BB[n].y));
+                    if (a && b)
+                        done = adj_add<AMP, true, 2>(sbase, r2, base, T2 + p, F4 + p, BB + p, MK + p);
+                    else if (b)
+                        done = adj_add<AMP, true, 1>(sbase, r2, base, T2 + n, F4 + n, BB + n, MK + n);
+                    else
+                        done = adj_add<AMP, true, 1>(sbase, r2, base, T2 + p, F4 + p, BB + p, MK + p);
+                }
+            }
+            if (!done) {
+#pragma unroll
+                for (int j = p; j <= n; ++j)
+                    adj_term2<AMP, true>(sbase, r2, base, smax, T2[j].x, F4[j].x, BB[j].x,
+                                         MK[j].x, T2[j].y, F4[j].y, BB[j].y, MK[j].y);
+                __syncwarp();
             }
         }
     }
@@ -254,12 +381,21 @@ __device__ __forceinline__ void adj_visit(unsigned char* sbase, float r2, uint32
 // in place (times 2^-s, exact below 2^53), and the data cube accumulates in FP64.
 template <bool FIX>
 __device__ __forceinline__ void adj_flush(const AdjParams& A, const AdjMeta& m,
-                                          unsigned char* stage, uint32_t smem_abs, int lane,
-                                          double inv_scale) {
+                                          unsigned char* stage, uint32_t stage_off,
+                                          uint32_t smem_abs, int lane, double inv_scale) {
     if (FIX) {
         long long* w = reinterpret_cast<long long*>(stage);
         for (int i = lane; i < m.tot; i += 32)
             reinterpret_cast<double*>(w)[i] = static_cast<double>(w[i]) * inv_scale;
+        __syncwarp();
+    }
+    if constexpr (!FIX) {  // nothing beyond the record
+        for (int k = lane; k < m.count; k += 32) {
+            const int4 gg = m.g[k];  // row, crossline, ws, size
+            float* w = reinterpret_cast<float*>(
+                stage + (static_cast<uint32_t>(m.m[k]) + 4u * gg.z + kMagic4 - stage_off));
+            for (int i = max(A.F.n_t - gg.z, 0); i < gg.w; ++i) w[i] = 0.0f;
+        }
         __syncwarp();
     }
     fence_proxy_async_smem();  // the shared-memory sums -> the async proxy
@@ -295,10 +431,10 @@ __device__ __forceinline__ void adj_flush(const AdjParams& A, const AdjMeta& m,
     __syncwarp();
 }
 
-// MINB: CTAs per SM the kernel is built for (the host gives 3-CTA launches 32 KB stages): the
-// kernel is bound by the latency of its shared-memory atomics, which more warps hide.
-// FIX: 64-bit fixed-point window sums and an FP64 data cube (A.data64); else fp32 atomics and
-// an fp32 data cube (A.data).
+// MINB: CTAs per SM the kernel is built for (the host gives 3-CTA launches 32 KB stages): more
+// warps hide the latency of the shared-memory additions.
+// FIX: 64-bit fixed-point window sums (atomics) and an FP64 data cube (A.data64); else fp32 sums
+// and an fp32 data cube (A.data).
 template <bool AMP, int MINB = 2, bool FIX = false>
 __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjParams A) {
     constexpr int EB = FIX ? 8 : 4;           // bytes of a window sample
@@ -320,8 +456,8 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
     const int x0 = blockIdx.x * kTX;
     const int T0 = static_cast<int>(gridDim.z - 1 - blockIdx.z) * kTT;
 
-    float T2[kJ], F4[kJ], BB[kJ], MK[kJ];
-    float gmax[2], gmin[2];
+    float2 T2[kJ / 2], F4[kJ / 2], BB[kJ / 2], MK[kJ / 2];
+    float gmax[2], gmin[2], safe[2];
     float warpmax = -1.0f;
     const int x = x0 + warp - 1;
     if (warp > 0) {
@@ -331,50 +467,107 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
         const float* mp = A.image + (static_cast<size_t>(jobi) * P.n_ox +
                                      (x < P.n_ox ? x : 0)) * P.n_t;
         float vmin = 3.0e38f, vmax = 0.0f, bmax = -1.0f, t0min = 3.0e38f, t0max = 0.0f;
-        // lane l holds samples T0 + 64 (j / 2) + 2 l + (j % 2): the 32 lanes of one block
-        // are two samples apart, so their trace samples (ds/dt0 = t0 / t >= cos(aperture)
-        // inside the aperture, 0.7 at 45 deg) fall on different window addresses, and the
-        // shared-memory atomics of one instruction do not collide (the forward's mapping,
-        // consecutive samples across lanes, puts about one lane in five on its neighbour's
-        // address, which halves the atomics' rate); groups of 4 blocks still span 128
-        // consecutive samples
+        // lane l holds samples T0 + 64 p + 2 l and the one after it: the lanes of one block
+        // are two samples apart, so their trace samples (ds/dt0 = t0 / t >= cos(aperture) inside
+        // the aperture of a constant Vrms, 0.7 at 45 deg) fall on different window addresses;
+        // couples of blocks span 128 consecutive samples
+        bool sane = true;  // every sample of the record has a Vrms
 #pragma unroll
-        for (int j = 0; j < kJ; ++j) {
-            const int t = T0 + 64 * (j >> 1) + 2 * lane + (j & 1);
-            float v = 0.0f, t0v = 0.0f, mv = 0.0f;
-            if (xvalid && t < P.n_t) {
-                v = __ldg(vp + t);
-                t0v = __ldg(P.t0 + t);
-                mv = __ldg(mp + t);
+        for (int p = 0; p < kJ / 2; ++p) {
+            float t2[2], f4[2], bj[2], mk[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int t = T0 + 64 * p + 2 * lane + k;
+                float v = 0.0f, t0v = 0.0f, mv = 0.0f;
+                if (xvalid && t < P.n_t) {
+                    v = __ldg(vp + t);
+                    t0v = __ldg(P.t0 + t);
+                    mv = __ldg(mp + t);
+                    sane = sane && v >= 1e-5f;
+                }
+                const PointConst pc = point_const(v, t0v, P.tan2);
+                const float b = pass_bound<false>(pc, P.inv_dt, P.ntm1f);
+                bj[k] = b;
+                mk[k] = 0.0f;
+                if (FIX) {
+                    t2[k] = 1.0f;
+                    f4[k] = 0.0f;
+                } else {
+                    // samples without terms keep the order of s (their addresses anchor a
+                    // neighbour's, their shares are zero)
+                    const bool in = xvalid && t < P.n_t;
+                    t2[k] = in ? fmaxf(pc.t0sq * P.idt2, 0.25f) : kBeyond;
+                    f4[k] = in && v >= 1e-5f ? pc.f4 * P.idt2 : 0.0f;
+                }
+                if (b >= 0.0f) {
+                    t2[k] = pc.t0sq * P.idt2;
+                    f4[k] = pc.f4 * P.idt2;
+                    mk[k] = AMP ? mv * __fdiv_rn(P.inv_dt, __fmul_rn(v, v)) : mv;
+                    vmin = fminf(vmin, v);
+                    vmax = fmaxf(vmax, v);
+                    bmax = fmaxf(bmax, b);
+                    t0min = fminf(t0min, t0v);
+                    t0max = fmaxf(t0max, t0v);
+                }
             }
-            const PointConst pc = point_const(v, t0v, P.tan2);
-            const float b = pass_bound<false>(pc, P.inv_dt, P.ntm1f);
-            T2[j] = 1.0f;
-            F4[j] = 0.0f;
-            MK[j] = 0.0f;
-            if (b >= 0.0f) {
-                T2[j] = pc.t0sq * P.idt2;
-                F4[j] = pc.f4 * P.idt2;
-                MK[j] = AMP ? mv * __fdiv_rn(P.inv_dt, __fmul_rn(v, v)) : mv;
-                vmin = fminf(vmin, v);
-                vmax = fmaxf(vmax, v);
-                bmax = fmaxf(bmax, b);
-                t0min = fminf(t0min, t0v);
-                t0max = fmaxf(t0max, t0v);
-            }
-            BB[j] = b;
+            T2[p] = make_float2(t2[0], t2[1]);
+            F4[p] = make_float2(f4[0], f4[1]);
+            BB[p] = make_float2(bj[0], bj[1]);
+            MK[p] = make_float2(mk[0], mk[1]);
         }
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            float mx = BB[4 * g], mn = BB[4 * g];
+        for (int h = 0; h < 2; ++h) {
+            const float2 u = BB[2 * h], w = BB[2 * h + 1];
+            gmax[h] = warp_max(fmaxf(fmaxf(u.x, u.y), fmaxf(w.x, w.y)));
+            gmin[h] = warp_min(fminf(fminf(u.x, u.y), fminf(w.x, w.y)));
+            warpmax = fmaxf(warpmax, gmax[h]);
+            safe[h] = -1.0f;
+            if (!FIX && gmax[h] >= 0.0f) {
+                // each gap between two lanes' first samples (the last lane's next is the
+                // couple's second block's first) has to be good up to the largest r^2 at which
+                // lanes on both sides of it have terms
+                float r = 3.0e38f;
+                const float u0 = fmaxf(u.x, u.y), w0 = fmaxf(w.x, w.y);
+                float pu = u0, pw = w0, su = u0, sw = w0;  // running maxima from either end
 #pragma unroll
-            for (int k = 1; k < 4; ++k) {
-                mx = fmaxf(mx, BB[4 * g + k]);
-                mn = fminf(mn, BB[4 * g + k]);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const float a = __shfl_up_sync(0xffffffffu, pu, o);
+                    const float b = __shfl_up_sync(0xffffffffu, pw, o);
+                    const float c = __shfl_down_sync(0xffffffffu, su, o);
+                    const float d = __shfl_down_sync(0xffffffffu, sw, o);
+                    if (lane >= o) {
+                        pu = fmaxf(pu, a);
+                        pw = fmaxf(pw, b);
+                    }
+                    if (lane + o < 32) {
+                        su = fmaxf(su, c);
+                        sw = fmaxf(sw, d);
+                    }
+                }
+                pw = fmaxf(pw, __shfl_sync(0xffffffffu, pu, 31));
+                su = fmaxf(su, __shfl_sync(0xffffffffu, sw, 0));
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float2 t2 = T2[2 * h + k], f4 = F4[2 * h + k];
+                    float tn = __shfl_down_sync(0xffffffffu, t2.x, 1);
+                    float fn = __shfl_down_sync(0xffffffffu, f4.x, 1);
+                    float after = __shfl_down_sync(0xffffffffu, k ? sw : su, 1);
+                    if (k == 0) {
+                        const float tb = __shfl_sync(0xffffffffu, T2[2 * h + 1].x, 0);
+                        const float fb = __shfl_sync(0xffffffffu, F4[2 * h + 1].x, 0);
+                        const float ab = __shfl_sync(0xffffffffu, sw, 0);
+                        if (lane == 31) {
+                            tn = tb;
+                            fn = fb;
+                            after = ab;
+                        }
+                    }
+                    const float top = fminf(k ? pw : pu, after);
+                    if ((lane < 31 || k == 0) && top >= 0.0f && t2.x < kBeyond)
+                        r = fminf(r, safe_reach(t2.x, f4.x, tn, fn, top));
+                }
+                safe[h] = __all_sync(0xffffffffu, sane) ? warp_min(r) : -1.0f;
             }
-            gmax[g] = warp_max(mx);
-            gmin[g] = warp_min(mn);
-            warpmax = fmaxf(warpmax, gmax[g]);
         }
         vmin = warp_min(vmin);
         vmax = warp_max(vmax);
@@ -383,7 +576,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
         t0max = warp_max(t0max);
         float mkm = 0.0f;
 #pragma unroll
-        for (int j = 0; j < kJ; ++j) mkm = fmaxf(mkm, fabsf(MK[j]));
+        for (int p = 0; p < kJ / 2; ++p) mkm = fmaxf(mkm, fmaxf(fabsf(MK[p].x), fabsf(MK[p].y)));
         mkm = warp_max(mkm);
         if (lane == 0) {
             TileStats s;
@@ -413,7 +606,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
         if (warp > 0) {
             const float sc = ldexpf(1.0f, shift);
 #pragma unroll
-            for (int j = 0; j < kJ; ++j) MK[j] *= sc;
+            for (int p = 0; p < kJ / 2; ++p) MK[p] = make_float2(MK[p].x * sc, MK[p].y * sc);
         }
     }
 
@@ -531,7 +724,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                 unsigned char* stage_ptr =
                     smem_raw + L.stage + static_cast<uint32_t>(EB) * stage * P.stage_cap;
                 if (it >= static_cast<uint32_t>(kStages))
-                    adj_flush<FIX>(A, m, stage_ptr, smem_abs, lane, inv_scale);
+                    adj_flush<FIX>(A, m, stage_ptr, stage_ptr - smem_raw, smem_abs, lane, inv_scale);
                 const int tot = __shfl_sync(0xffffffffu, take ? cum : 0, consumed - 1);
                 // zero the accumulator region of the new windows (16 B per lane per step;
                 // windows are 16-byte multiples)
@@ -575,6 +768,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                 if (it >= static_cast<uint32_t>(kStages))
                     adj_flush<FIX>(A, meta[stage],
                                    smem_raw + L.stage + static_cast<uint32_t>(EB) * stage * P.stage_cap,
+                                   L.stage + static_cast<uint32_t>(EB) * stage * P.stage_cap,
                                    smem_abs, lane, inv_scale);
                 if (lane == 0) {
                     meta[stage].count = -1;
@@ -590,6 +784,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     if (__shfl_sync(0xffffffffu, ok2, 0))
                         adj_flush<FIX>(A, meta[s2],
                                        smem_raw + L.stage + static_cast<uint32_t>(EB) * s2 * P.stage_cap,
+                                       L.stage + static_cast<uint32_t>(EB) * s2 * P.stage_cap,
                                        smem_abs, lane, inv_scale);
                 }
             }
@@ -599,21 +794,41 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
     }
 
     // -------------------------------------------------------------------- consumers
+    // fp32 sums: the stage's slots are dealt into kTX groups, and the warps take the groups in
+    // turn (warp w group w + step), with a barrier after each step, so that one warp at a time
+    // adds into a window and no atomics are needed: a shared fp32 atomic is a compare-and-swap
+    // loop of about 6 wavefronts here, a load and a store are 4.
     uint32_t it = 0;
     while (true) {
         const int stage = it % kStages;
         const uint32_t par = (it / kStages) & 1u;
-        if (!mbar_wait(&full[stage], par, P.err, P.wait_us)) break;
+        bool ok = mbar_wait(&full[stage], par, P.err, P.wait_us);
+        if (!FIX) ok = consumers_agree(ok);  // (the steps' barriers need every warp)
+        if (!ok) break;
         const AdjMeta& m = meta[stage];
         const int cnt = m.count;
         if (cnt < 0) break;
-        for (int g = 0; g < cnt; ++g) {
-            const float r2 = m.r2[g][warp - 1];
-            if (r2 > warpmax) continue;
-            adj_visit<AMP, FIX>(smem_raw, r2, static_cast<uint32_t>(m.m[g]), P.ntm1m, gmax, gmin,
-                                T2, F4, BB, MK);
+        if constexpr (FIX) {
+            for (int g = 0; g < cnt; ++g) {
+                const float r2 = m.r2[g][warp - 1];
+                if (r2 > warpmax) continue;
+                adj_visit_fixed<AMP>(smem_raw, r2, static_cast<uint32_t>(m.m[g]), P.ntm1m, gmax,
+                                     gmin, T2, F4, BB, MK);
+            }
+            __syncwarp();
+        } else {
+            for (int step = 0; step < kTX; ++step) {
+                // (every kTX-th slot: neighbouring slots have similar work)
+                for (int g = (warp - 1 + step) % kTX; g < cnt; g += kTX) {
+                    const float r2 = m.r2[g][warp - 1];
+                    if (r2 > warpmax) continue;
+                    adj_visit<AMP>(smem_raw, r2, static_cast<uint32_t>(m.m[g]), P.ntm1m, gmax,
+                                   gmin, safe, T2, F4, BB, MK);
+                }
+                if (step + 1 < kTX) consumer_barrier();
+            }
+            __syncwarp();
         }
-        __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         ++it;
     }
