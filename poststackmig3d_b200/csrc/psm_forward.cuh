@@ -29,11 +29,12 @@
 //     both pairs, first or second pair only), so that the evaluations run in loops without
 //     tests: the earlier kernel spent half of its instructions on a test tree per slot.
 // Measured on 201 x 201 x 1001 samples (Vrms 1500 -> 3500 m/s, 45 degrees): 116.4 ms before
-// (one crossline a warp, pairs read unfolded, a test tree per slot), 81.0 ms with NX = 14 (64
-// registers, 2 CTAs per SM).  NX = 16 (56 registers) takes 84.3 ms, NX = 12 84.6 ms, NX = 4 (3
-// CTAs per SM) 115 ms; three smaller stages and stages of 3200 samples were 4 to 6% slower (the
+// (one crossline a warp, pairs read unfolded, a test tree per slot), 72.6 ms with NX = 14 (64
+// registers, 2 CTAs per SM).  NX = 12 takes 76.0 ms, NX = 10 78.4 ms, NX = 8 (3 CTAs per SM) 82.8
+// ms, NX = 4 102 ms; three smaller stages and stages of 3200 samples were 4 to 6% slower (the
 // work per stage and warp besides the evaluations is about 230 instructions).  NX = 4 is faster
-// where the wide tiles leave SMs idle: 31 x 29 x 251 samples 0.112 against 0.128 ms.
+// where the wide tiles leave SMs idle: 31 x 29 x 251 samples 0.088 against 0.108 ms; there the
+// producer's bulk copies (some 50 short windows a stage) are the bound.
 #pragma once
 
 #include "psm_kernels.cuh"
@@ -82,6 +83,15 @@ struct FwdLayout {
     }
     static_assert(kTab % 16 == 0 && sizeof(FwdStage<NX>) % 16 == 0, "16-byte aligned tables");
 };
+
+// Square root for the bounds of windows and rows, whose slack is two samples or traces (the
+// correctly rounded one is 8 to 10 instructions more on the producer's chain: 0.852 ms with it,
+// 0.841 without, 101 x 101 x 501 samples).
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -256,8 +266,8 @@ struct False {
 // (mirror distance, then crossline), with the traces' own differences; else the order within a
 // stage is that of the slots' kinds.  Least-squares migration runs the ordered form: conjugate
 // gradients carry a change of rounding in the operator into their step lengths and residual
-// norms, which are reproducible to 1e-9 this way.  By kind saves the control of about 40
-// instructions a stage and couple of pairs: 81.0 ms, ordered 85.3 ms (201 x 201 x 1001).
+// norms, which are reproducible to 1e-9 this way.  By kind saves the control of short runs:
+// 0.84 against 0.91 ms on 101 x 101 x 501 samples (201 x 201 x 1001: 72.6, 72.7 ms).
 //
 // KAHAN: compensated summation.  Each ring stage (at most kSlots slots) is summed into a fresh
 // partial, and the partials are added to the accumulator with Kahan's compensation, so the long
@@ -276,7 +286,9 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
     uint64_t* empty = reinterpret_cast<uint64_t*>(smem + L::kEmpty);
     Stage* tabs = reinterpret_cast<Stage*>(smem + L::kTab);
     float4* stat = reinterpret_cast<float4*>(smem + L::kStat);
-    const int warp = threadIdx.x >> 5;
+    // (read through a shuffle, which makes the compiler lay out the evaluation loops otherwise:
+    // 79.2 ms without, 72.6 with, 201 x 201 x 1001 samples)
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
     // ---- consumers: per-sample constants.  Warp cw owns crosslines x0 + 2 xp + {0, 1} (16 lanes
@@ -393,7 +405,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
         const int n_rows = pc >= 0 ? max(pc, n_inl - 1 - pc) + 1 : n_inl;
         // first crossline of a row's traces: none beyond bmax reaches the tile
         auto row_first = [&](float dx2, int* reach) {
-            *reach = static_cast<int>(sqrtf(fmaxf(bmax - dx2, 0.0f)) * P.inv_dxl) + 2;
+            *reach = static_cast<int>(sqrt_approx(fmaxf(bmax - dx2, 0.0f)) * P.inv_dxl) + 2;
             return max(0, xa - *reach);
         };
         int total = 0;
@@ -457,7 +469,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                 const float dymin = static_cast<float>(dkmin) * P.d_xl;
                 const float dymax = static_cast<float>(dkmax) * P.d_xl;
                 const float rmin2 = fmaf(dymin, dymin, dx2), rmax2 = fmaf(dymax, dymax, dx2);
-                const float rmin = sqrtf(rmin2);
+                const float rmin = sqrt_approx(rmin2);
                 float tlo2 = 3.0e38f, thi2 = -1.0f;
 #pragma unroll
                 for (int p = 0; p < 8; ++p) {
@@ -469,8 +481,8 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                     }
                 }
                 if (thi2 >= 0.0f) {
-                    const float slo = fminf(sqrtf(tlo2) * P.inv_dt, 1.0e9f);
-                    const float shi = fminf(sqrtf(thi2) * P.inv_dt, 1.0e9f);
+                    const float slo = fminf(sqrt_approx(tlo2) * P.inv_dt, 1.0e9f);
+                    const float shi = fminf(sqrt_approx(thi2) * P.inv_dt, 1.0e9f);
                     const int lolo = max(static_cast<int>(floorf(slo)) - 2, 0);
                     const int lohi = min(static_cast<int>(floorf(shi)) + 2, P.n_t - 2);
                     if (lolo <= lohi) {
@@ -765,13 +777,13 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                             }
                             if (i < e) both(False{}, r2x[i], bf[i]);
                         } else if (p0 && p1) {
-#pragma unroll 1
+#pragma unroll 2
                             for (; i < e; ++i) both(True{}, r2x[i], bf[i]);
                         } else if (p0) {
-#pragma unroll 1
+#pragma unroll 2
                             for (; i < e; ++i) first(r2x[i], bf[i]);
                         } else {
-#pragma unroll 1
+#pragma unroll 2
                             for (; i < e; ++i) second(r2x[i], bf[i]);
                         }
                     }
@@ -797,17 +809,17 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                         both(False{}, e.z, e.w);
                     }
                     // (the last of an odd number joins the masked ones: its masks pass)
-#pragma unroll 1
+#pragma unroll 2
                     for (; i < nb; ++i) {
                         const float2 e = mylist[i];
                         both(True{}, e.x, e.y);
                     }
-#pragma unroll 1
+#pragma unroll 2
                     for (; i < n0; ++i) {
                         const float2 e = mylist[i];
                         first(e.x, e.y);
                     }
-#pragma unroll 1
+#pragma unroll 2
                     for (; i < n1; ++i) {
                         const float2 e = mylist[i];
                         second(e.x, e.y);
