@@ -909,8 +909,10 @@ int psm_set_vrms_table(psm_ctx* c, const int32_t* p_il, const int32_t* p_xl,
     PSM_CUDA_TRY(c->st, upload(d_v, p_v, n_points, s));
     PSM_CUDA_TRY(c->st, upload(d_lil, il_labels, c->g.n_il, s));
     PSM_CUDA_TRY(c->st, upload(d_lxl, xl_labels, c->g.n_xl, s));
-    const size_t n = static_cast<size_t>(c->g.n_il) * c->g.n_xl * c->g.n_t;
-    psm::vrms_table_kernel<<<vrms_blocks(n), 256, 0, s>>>(
+    const size_t n_items = static_cast<size_t>(c->g.n_il) * c->g.n_xl *
+                           ((c->g.n_t + psm::kTableThreads - 1) / psm::kTableThreads);
+    const unsigned grid = static_cast<unsigned>(std::min<size_t>(n_items, 148 * 64));
+    psm::vrms_table_kernel<<<grid, psm::kTableThreads, 0, s>>>(
         d_il.as<int32_t>(), d_xl.as<int32_t>(), d_t.as<double>(), d_v.as<float>(), n_points,
         vmin, d_lil.as<int32_t>(), d_lxl.as<int32_t>(), c->g.n_il, c->g.n_xl, c->g.n_t,
         c->g.dt_seconds, c->vrms.as<float>());

@@ -15,46 +15,102 @@
 
 namespace psm {
 
+constexpr int kTableThreads = 128;  // samples of a work item
+constexpr int kTablePoints = 64;    // table points staged in shared memory at a time
+
+// float(sqrt(x)) for the double x, as rounding to double first and to float then gives it; clears
+// *sure when the caller has to take the exact root.  Two Newton steps from an approximate
+// 1 / sqrt(x) (off by 2^-19 at the worst) leave 4 units of the double's last place at most, so
+// float(s) is the wanted float unless s lies about the middle between two floats (32 units
+// here), or x is too small (an exact hit may be) or large for the steps.
+__device__ __forceinline__ float root_to_float(double x, bool* sure) {
+    double q;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(x));
+    const double h = __dmul_rn(0.5, q), y = __dmul_rn(x, q);
+    const double r = __fma_rn(__fma_rn(-y, y, x), h, y);
+    const double s = __fma_rn(__fma_rn(-r, r, x), h, r);
+    constexpr unsigned kMiddle = 1u << 28, kNear = 32u;
+    constexpr unsigned kLo = 0x3c400000u, kHi = 0x47000000u;  // high words of 2^-59 and 2^113
+    const unsigned low = static_cast<unsigned>(__double2loint(s)) & (2u * kMiddle - 1u);
+    *sure &= (low - (kMiddle - kNear) > 2u * kNear) &
+             (static_cast<unsigned>(__double2hiint(x)) - kLo < kHi - kLo);
+    return __double2float_rn(s);
+}
+
 // Text-table Vrms: every point (il, xl, time, v) weighted by 1 / (1 + dist) with dist mixing
 // label units and seconds; an exact hit (dist < 1e-10) returns that point's v; a result <= 0
 // (or no weight) gives vmin.  out [n_il][n_xl][n_t], t0 = t * dt.
-__global__ void vrms_table_kernel(const int32_t* __restrict__ p_il,
-                                  const int32_t* __restrict__ p_xl,
-                                  const double* __restrict__ p_time,
-                                  const float* __restrict__ p_v, int n_points, float vmin,
-                                  const int32_t* __restrict__ il, const int32_t* __restrict__ xl,
-                                  int n_il, int n_xl, int n_t, double dt,
-                                  float* __restrict__ out) {
-    const int64_t n = static_cast<int64_t>(n_il) * n_xl * n_t;
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
-         k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int t = static_cast<int>(k % n_t);
-        const int64_t tr = k / n_t;
+//
+// Bound by instructions, some 45 per point and sample (84% of the issue slots).  A work item is
+// kTableThreads samples of one trace; the label part of the squared distances is summed once per
+// item and point; a thread whose root_to_float was not sure of one of the staged points (an
+// exact hit, or 1 in 2^23) takes those points again with the exact root.
+// 81 x 93 x 626 samples, 54 points: 659 us with the exact root and divide everywhere, 466 us with
+// a branch to the exact root per point (and one Newton step), 397 us so.
+__global__ void __launch_bounds__(kTableThreads)
+vrms_table_kernel(const int32_t* __restrict__ p_il, const int32_t* __restrict__ p_xl,
+                  const double* __restrict__ p_time, const float* __restrict__ p_v, int n_points,
+                  float vmin, const int32_t* __restrict__ il, const int32_t* __restrict__ xl,
+                  int n_il, int n_xl, int n_t, double dt, float* __restrict__ out) {
+    __shared__ double2 at[kTablePoints];  // label part of the squared distance, time
+    __shared__ float vel[kTablePoints];
+    const int n_seg = (n_t + kTableThreads - 1) / kTableThreads;
+    const int64_t n_items = static_cast<int64_t>(n_il) * n_xl * n_seg;
+    for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int64_t tr = item / n_seg;
+        const int t = static_cast<int>(item % n_seg) * kTableThreads + threadIdx.x;
         const int32_t a_il = il[tr / n_xl], a_xl = xl[tr % n_xl];
         const double time = __dmul_rn(static_cast<double>(t), dt);
         float sv = 0.0f, sw = 0.0f, hit_v = 0.0f;
         bool hit = false;
-        for (int p = 0; p < n_points; ++p) {
-            const double a = fabs(static_cast<double>(p_il[p] - a_il));
-            const double b = fabs(static_cast<double>(p_xl[p] - a_xl));
-            const double c = fabs(__dsub_rn(p_time[p], time));
-            const double d =
-                __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c)));
-            if (d < 1e-10) {
-                hit = true;
-                hit_v = p_v[p];
-                break;
+        for (int base = 0; base < n_points; base += kTablePoints) {
+            const int cnt = min(kTablePoints, n_points - base);
+            __syncthreads();  // the readers of the points before these
+            for (int p = threadIdx.x; p < cnt; p += kTableThreads) {
+                const double a = fabs(static_cast<double>(p_il[base + p] - a_il));
+                const double b = fabs(static_cast<double>(p_xl[base + p] - a_xl));
+                at[p] = make_double2(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)),
+                                     p_time[base + p]);
+                vel[p] = p_v[base + p];
             }
-            const float w = __fdiv_rn(1.0f, __fadd_rn(1.0f, __double2float_rn(d)));
-            sv = __fadd_rn(sv, __fmul_rn(p_v[p], w));
-            sw = __fadd_rn(sw, w);
+            __syncthreads();
+            if (t >= n_t || hit) continue;
+            const float v0 = sv, w0 = sw;
+            bool sure = true;
+#pragma unroll 2
+            for (int p = 0; p < cnt; ++p) {
+                const double2 u = at[p];
+                const double c = __dsub_rn(u.y, time);
+                const float d = root_to_float(__dadd_rn(u.x, __dmul_rn(c, c)), &sure);
+                const float w = __frcp_rn(__fadd_rn(1.0f, d));
+                sv = __fadd_rn(sv, __fmul_rn(vel[p], w));
+                sw = __fadd_rn(sw, w);
+            }
+            if (sure) continue;
+            sv = v0;  // again, with the exact root
+            sw = w0;
+#pragma unroll 1
+            for (int p = 0; p < cnt; ++p) {
+                const double2 u = at[p];
+                const double c = __dsub_rn(u.y, time);
+                const double d = __dsqrt_rn(__dadd_rn(u.x, __dmul_rn(c, c)));
+                if (d < 1e-10) {
+                    hit = true;
+                    hit_v = vel[p];
+                    break;
+                }
+                const float w = __fdiv_rn(1.0f, __fadd_rn(1.0f, __double2float_rn(d)));
+                sv = __fadd_rn(sv, __fmul_rn(vel[p], w));
+                sw = __fadd_rn(sw, w);
+            }
         }
+        if (t >= n_t) continue;
         float r = hit_v;
         if (!hit) {
             r = sw > 0.0f ? __fdiv_rn(sv, sw) : vmin;
             if (r <= 0.0f) r = vmin;
         }
-        out[k] = r;
+        out[tr * n_t + t] = r;
     }
 }
 

@@ -88,3 +88,23 @@ def test_grid_vrms_matches_host_and_reference(tmp_path, kind):
         np.testing.assert_allclose(got, ref, rtol=4e-7, atol=0)
     else:
         assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("n_points,n_t", [(1, 1), (63, 127), (64, 128), (65, 129), (200, 300)])
+def test_table_vrms_chunks_and_segments(tmp_path, n_points, n_t):
+    """Edges of the staged points (64) and of the work items (128 samples), with exact hits,
+    points too close for the fast root and labels far away.  Equal bits."""
+    rng = np.random.default_rng(n_points)
+    il = np.array([3, 4, 2_000_000_000], dtype=np.int32)
+    xl = np.array([8, 1_000_000], dtype=np.int32)
+    pts = [(int(rng.choice(il[:2])), int(rng.integers(1, 20)),
+            float(rng.integers(0, n_t + 1) * 0.002 + rng.choice([0.0, 3e-11, 2e-9, 1e-6, 1e-3])),
+            float(np.float32(rng.uniform(1500, 3500)))) for _ in range(n_points)]
+    pts[-1] = (4, 8, (n_t - 1) * 0.002, 2222.0)  # the last point hits the last sample
+    t = tmp_path / "t.txt"
+    t.write_text("".join(f"{a} {b} {c!r} {d!r}\n" for a, b, c, d in pts))
+    host = H.velocity_cube(str(t), il, xl, n_t, 0.002)
+    with _migrator(il, xl, n_t, 0.002) as m:
+        m.set_vrms_table(pts, il, xl)
+        got = m.get_vrms()
+    assert np.array_equal(got, host)
