@@ -41,22 +41,22 @@ METRIC = ("summed input samples/s (G/s) on 1 B200, mixed/batched vs plain FP32 a
           "rel err")
 UNIT = "G/s"
 # Algorithmic needs of one term (an output sample and an input trace that pass the masks) on
-# the SM limbs: one load of the staged sample pair (both interpolation operands: 8 bytes in
-# fp32 storage, 4 in 16-bit storage), one rsqrt (travel time and weight; mirrored pairs share
-# it between two traces, so half), and the fp32 lane operations of t^2, s, floor, frac, the
-# interpolation and the weighted accumulate (7; 4.5 with pairs, which add the two traces'
-# samples and interpolate once).  Peak terms/s = min over limbs of (measured rate per clock
-# per SM / need per term) x SMs x SM clock; the limbs come from psm_measure_limbs.
-FP32_OPS_PER_TERM = {False: 7.0, True: 4.5}
+# the SM limbs: one 8-byte shared load of both interpolation operands, one rsqrt (travel time
+# and weight), and the fp32 lane operations of t^2, s, floor, frac, the interpolation and the
+# weighted accumulate (7).  A mirrored pair of traces is folded into one window, so it needs
+# them once for two terms.  Peak terms/s = min over limbs of (measured rate per clock per SM
+# / need per term) x SMs x SM clock; the limbs come from psm_measure_limbs.
+FP32_OPS_PER_TERM = {False: 7.0, True: 3.5}
+LOAD_BYTES_PER_TERM = {False: 8.0, True: 4.0}
 N_SM = 148
 
 
-def limb_roofline(limbs, sm_mhz, achieved_gterms, paired, elem_bytes):
+def limb_roofline(limbs, sm_mhz, achieved_gterms, paired):
     """Roofline of the summation over the measured limbs: {bound, peak (Gterm/s), per-limb
     peaks and needs}."""
     n_sm = int(limbs.get("n_sm") or N_SM)
     per = {
-        "lds": (limbs["lds64_bytes_per_clk_sm"], float(elem_bytes), "B"),
+        "lds": (limbs["lds64_bytes_per_clk_sm"], LOAD_BYTES_PER_TERM[bool(paired)], "B"),
         "mufu": (limbs["rsqrt_per_clk_sm"], 0.5 if paired else 1.0, "rsqrt"),
         "fp32": (max(limbs["ffma_per_clk_sm"], limbs["ffma2_per_clk_sm"]),
                  FP32_OPS_PER_TERM[bool(paired)], "lane-ops"),
@@ -498,8 +498,7 @@ def run_ours(args):
     sm_mhz = clocks["sm_mhz"] or limbs["sm_clock_mhz"]
     achieved = n_terms_local / (ms * 1e-3) / 1e9  # this GPU's launch
     paired = "pairs" in Migrator.VARIANTS[m.variant()]
-    bound, peak, limb_peaks = limb_roofline(limbs, sm_mhz, achieved, paired,
-                                            8 if g.precision == "f32" else 4)
+    bound, peak, limb_peaks = limb_roofline(limbs, sm_mhz, achieved, paired)
     comp_bytes = (2 * g.n_il * g.n_xl * g.n_t + g.n_oi * g.n_ox * g.n_t) * 4
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -665,8 +664,8 @@ def run_lsm(args):
                 "terms_per_application": n_terms, "forward_ms": fwd_ms, "adjoint_ms": adj_ms,
                 "adjoint_gterm_s": n_terms / (adj_ms * 1e-3) / 1e9,
                 "adjoint_roofline": {
-                    "bound": "shared fp32 atomics (one per term: a mirrored pair of traces "
-                             "shares one window)",
+                    "bound": "shared fp32 atomics (one per term; the kernel adds without them, "
+                             "so this is a rate to compare with, not a limit)",
                     "achieved": n_terms / (adj_ms * 1e-3) / 1e9,
                     "peak": limbs["atom_per_clk_sm"] * limbs["n_sm"] * limbs["sm_clock_mhz"]
                             * 1e6 / 1e9,
@@ -819,8 +818,7 @@ def run_batch(args):
                       ", fed the dequantised samples" if args.storage != "f32" else "")}
     sm_mhz = clocks["sm_mhz"] or limbs["sm_clock_mhz"]
     bound, peak, limb_peaks = limb_roofline(limbs, sm_mhz, value,
-                                            "pairs" in Migrator.VARIANTS[b.variant()],
-                                            8 if args.storage == "f32" else 4)
+                                            "pairs" in Migrator.VARIANTS[b.variant()])
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": 1, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32",
