@@ -18,7 +18,7 @@
 // output inline c) have the same r^2 to every output point, hence the same travel times,
 // fractions and weights: every term adds the same two shares to both.  They share one slot
 // and ONE window, which the flush adds into both traces (two bulk reductions of the same
-// shared-memory window), so a pair costs the atomics of a single trace.
+// shared-memory window), so a pair costs the additions of a single trace.
 #pragma once
 
 #include "psm_kernels.cuh"
@@ -33,7 +33,7 @@ static_assert(kTX == 8 && kMaxG == 32, "a lane per slot; kEveryTX");
 constexpr unsigned kEveryTX = 0x01010101u;  // slots 0, kTX, 2 kTX, ...
 
 struct AdjParams {
-    FwdParams F;          // geometry, tables, constants (F.pairs unused)
+    FwdParams F;          // geometry, tables, constants (F.traces unused)
     const float* image;   // [n_jobs][n_ox][n_t]: image of each job (duplicate rows folded)
     float* data;          // [n_ci][n_cx][ns] accumulated in place (zero it first)
     double* data64;       // fixed-point form: [n_ci][n_cx][ns] accumulated in FP64 instead
@@ -145,13 +145,13 @@ __device__ __forceinline__ void adj_window(const FwdParams& P, const TileStats& 
     *size_out = we - ws;
 }
 
-// One term of the transpose (scalar FP32) for a slot: the forward's s, frac and q, then two
+// One term of the transpose for a slot, fixed-point form: the forward's s, frac and q, then two
 // atomic adds into the slot's window.  A failing term (MASK) returns before touching memory;
 // a passing term's lo lies in its window (adj_window), with s held below n_t - 1 (smax) so
 // that lo + 1 stays on the trace.
-// FIX: MK is m K in units of 2^-s (exact power-of-two scaling); the shares go into the
-// window as 64-bit integers (rounded to nearest).
-template <bool AMP, bool MASK, bool FIX>
+// MK is m K in units of 2^-s (exact power-of-two scaling); the shares go into the window as
+// 64-bit integers (rounded to nearest).
+template <bool AMP, bool MASK>
 __device__ __forceinline__ void adj_term(unsigned char* sbase, float r2, uint32_t base,
                                          float smax, float T2, float F4, float BB, float MK) {
     const float t2 = __fmaf_rn(F4, r2, T2);
@@ -163,20 +163,12 @@ __device__ __forceinline__ void adj_term(unsigned char* sbase, float r2, uint32_
     const float c = AMP ? MK * q : MK;
     const float c1 = c * fr;
     const float c0 = c - c1;
-    if (FIX) {
-        unsigned long long* p = reinterpret_cast<unsigned long long*>(
-            sbase + (base + (__float_as_uint(mm) << 3)));
-        atomicAdd(p, static_cast<unsigned long long>(__float2ll_rn(c0)));
-        atomicAdd(p + 1, static_cast<unsigned long long>(__float2ll_rn(c1)));
-    } else {
-        float* p = reinterpret_cast<float*>(sbase + (base + (__float_as_uint(mm) << 2)));
-        atomicAdd(p, c0);
-        atomicAdd(p + 1, c1);
-    }
+    unsigned long long* p =
+        reinterpret_cast<unsigned long long*>(sbase + (base + (__float_as_uint(mm) << 3)));
+    atomicAdd(p, static_cast<unsigned long long>(__float2ll_rn(c0)));
+    atomicAdd(p + 1, static_cast<unsigned long long>(__float2ll_rn(c1)));
 }
 
-// One slot for one consumer warp: the groups of blocks where some lane passes, without masks
-// where every lane of the group passes.
 // Two terms of one lane for a slot: samples t and t + 1 (blocks j and j + 1), fp32 sums.
 // With ds/dt0 <= 1 their floor(s) are equal or adjacent, so their four shares fall on at
 // most three window addresses: lo_a (c0_a), lo_a + 1 (c1_a, and c0_b when lo_b = lo_a + 1),
@@ -214,6 +206,8 @@ __device__ __forceinline__ void adj_term2(unsigned char* sbase, float r2, uint32
     }
 }
 
+// One slot for one consumer warp, fixed-point form: the couples of blocks where some lane passes,
+// without masks where every lane of the couple passes.
 template <bool AMP>
 __device__ __forceinline__ void adj_visit_fixed(unsigned char* sbase, float r2, uint32_t base,
                                                 float smax, const float (&gmax)[2],
@@ -227,14 +221,14 @@ __device__ __forceinline__ void adj_visit_fixed(unsigned char* sbase, float r2, 
 #pragma unroll
             for (int p = 2 * h; p < 2 * h + 2; ++p) {
                 if (r2 <= gmin[h]) {
-                    adj_term<AMP, false, true>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
+                    adj_term<AMP, false>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
                                                MK[p].x);
-                    adj_term<AMP, false, true>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
+                    adj_term<AMP, false>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
                                                MK[p].y);
                 } else {
-                    adj_term<AMP, true, true>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
+                    adj_term<AMP, true>(sbase, r2, base, smax, T2[p].x, F4[p].x, BB[p].x,
                                               MK[p].x);
-                    adj_term<AMP, true, true>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
+                    adj_term<AMP, true>(sbase, r2, base, smax, T2[p].y, F4[p].y, BB[p].y,
                                               MK[p].y);
                 }
             }

@@ -402,7 +402,7 @@ struct psm_ctx {
     // that order staging, placement and the image copies
     DevBuf str_tr, str_v, str_img[2];
     cudaEvent_t ev_placed = nullptr, ev_staged = nullptr, ev_done[2] = {nullptr, nullptr};
-    // adjoint: 64-bit fixed-point window sums and an FP64 data cube (else fp32 atomics)
+    // adjoint: 64-bit fixed-point window sums and an FP64 data cube (else fp32 sums)
     bool adj_fixed = false;
     DevBuf adj64;
     // limit of the kernels' mbarrier waits (us; 0: the kernels' default of 4 s) and the

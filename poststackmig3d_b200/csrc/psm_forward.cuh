@@ -17,7 +17,7 @@
 // evaluation (64 output samples of one slot) needs 2 rsqrt warp instructions (16 cycles of a
 // sub-partition's XU), 6 packed and 2 scalar FMA instructions and 2 addresses (16 to 18 cycles
 // of its FMA pipe) and 4 wavefronts of shared loads (16 cycles of a quarter of the SM), so the
-// three pipes are about equally loaded; the loop alone runs at 22 cycles an evaluation.
+// three pipes are about equally loaded; the loop runs at 20 to 21 cycles an evaluation.
 // Reasons for the layout:
 //   * folding a pair before the consumers read it halves their shared loads and takes one
 //     packed add a load away; a window of about 150 samples is read by NX crosslines, so the
