@@ -349,6 +349,23 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             }
         }
     }
+    // The producer's share of the wait: smallest and largest t0 of each block of 32 samples (lane
+    // b holds block b), whatever their order (the per-inline call takes the caller's times).
+    // A sample has terms only with t0 > 0; every other counts as 0.
+    float t0min = 0.0f, t0max = 0.0f;
+    if (warp == 0) {
+#pragma unroll
+        for (int b = 0; b < kTileT / 32; ++b) {
+            const float t = __ldg(P.t0 + min(T0 + 32 * b + lane, P.n_t - 1));
+            const int bits = t > 0.0f ? __float_as_int(t) : 0;
+            const int mn = __reduce_min_sync(0xffffffffu, bits);
+            const int mx = __reduce_max_sync(0xffffffffu, bits);
+            if (lane == b) {
+                t0min = __int_as_float(mn);
+                t0max = __int_as_float(mx);
+            }
+        }
+    }
     __syncthreads();
 
     if (warp == 0) {
@@ -356,8 +373,8 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
         const int store = P.store, rb = store_bytes(store);
         const int A = store == kStoreBF16 || store == kStoreF16 ? 8 : 4;  // window alignment
         // bounds of each block of 32 samples over the tile's crosslines, in two float4: (largest
-        // B, first t0, 2 / (v_max tan), 4 / v_max^2), (last t0^2, 4 / v_min^2, last t0^2 (1 +
-        // tan^2), 1 when a sample passes)
+        // B, smallest t0, 2 / (v_max tan), 4 / v_max^2), (largest t0^2, 4 / v_min^2, largest t0^2
+        // (1 + tan^2), 1 when a sample passes)
         float4* blk = reinterpret_cast<float4*>(smem + L::kBlk);
         float bmax;
         {
@@ -376,15 +393,13 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             }
             bmax = warp_max(bmx);
             if (lane < 8) {
-                const float t0a = P.t0[min(T0 + 32 * lane, P.n_t - 1)];
-                const float t0b = P.t0[min(T0 + 32 * lane + 31, P.n_t - 1)];
                 blk[2 * lane] = make_float4(
-                    bmx * 1.0001f + 1e-6f, t0a,
+                    bmx * 1.0001f + 1e-6f, t0min,
                     P.tanth > 0.0f && vmx > 0.0f ? 2.0f / (vmx * P.tanth) : 0.0f,
                     4.0f / fmaf(vmx, vmx, 1e-10f));
-                blk[2 * lane + 1] =
-                    make_float4(t0b * t0b, 4.0f / fmaf(vmn, vmn, 1e-10f),
-                                t0b * t0b * (1.0f + P.tan2) * 1.0001f, bmx >= 0.0f ? 1.0f : 0.0f);
+                blk[2 * lane + 1] = make_float4(
+                    t0max * t0max, 4.0f / fmaf(vmn, vmn, 1e-10f),
+                    t0max * t0max * (1.0f + P.tan2) * 1.0001f, bmx >= 0.0f ? 1.0f : 0.0f);
             }
             __syncwarp();
         }
@@ -463,7 +478,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                 rowb = b >= 0 ? job.i0 + b : -1;
                 // window: over the blocks that the trace can reach, t^2 lies in [e^2 + 4 r_min^2 /
                 // v_max^2, min(t0^2 + 4 r_max^2 / v_min^2, t0^2 (1 + tan^2))] with e the later of
-                // the block's first t0 and the aperture's entry 2 r_min / (v_max tan)
+                // the block's smallest t0 and the aperture's entry 2 r_min / (v_max tan)
                 const int dkmin = kc < xa ? xa - kc : (kc > xb ? kc - xb : 0);
                 const int dkmax = max(abs(kc - xa), abs(kc - xb));
                 const float dymin = static_cast<float>(dkmin) * P.d_xl;
