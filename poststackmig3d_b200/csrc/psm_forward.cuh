@@ -699,6 +699,9 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             ++it;
             break;
         }
+#ifdef PSM_DEBUG_BOUNDS
+        const DebugWin dbg{m.base, m.win, n, P.err};
+#endif
         if (m.split) {  // part of one window: its terms one at a time
             const float r2 = m.r2[2 * xp + xl][0];
             const uint32_t base = static_cast<uint32_t>(m.base[0]);
@@ -710,8 +713,11 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                 const float mm = __fadd_rd(s, 8388608.0f);
                 const float lo = mm - 8388608.0f;
                 if (r2 <= b && lo >= slo && lo < shi) {
-                    const float2 a = *reinterpret_cast<const float2*>(
-                        smem + (base + (__float_as_uint(mm) << 3)));
+                    uint32_t o = base + (__float_as_uint(mm) << 3);
+#ifdef PSM_DEBUG_BOUNDS
+                    o = debug_check(dbg, base, o, L::kZero);
+#endif
+                    const float2 a = *reinterpret_cast<const float2*>(smem + o);
                     const float v = fmaf(s - lo, a.y, a.x);
                     const float add = AMP ? v * q : v;
                     if (KAHAN) {
@@ -730,9 +736,6 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             }
         } else {
             const float* r2x = m.r2[2 * xp + xl];
-#ifdef PSM_DEBUG_BOUNDS
-            const DebugWin dbg{m.base, m.win, n, P.err};
-#endif
             const bool in = lane < n;
             const float ra = in ? m.r2[2 * xp][lane] : 3.0e38f;
             const float rb = in ? m.r2[2 * xp + 1][lane] : 3.0e38f;
