@@ -183,13 +183,15 @@ auto grid_kernel() {
     return psm::fwd_kernel<K::AMP, K::KAHAN, K::ORDERED, K::NX, K::CAP, K::MINB>;
 }
 
-// A kernel's shared-memory limit.  It belongs to the kernel, so before a stream capture it is
-// set to cover the largest launch of the capture.
+// Lets a kernel be launched with `smem` bytes of dynamic shared memory.  The limit belongs to the
+// kernel, which other host threads launch with other amounts, so it is set to the same value on
+// every call: all that a CTA can have, less `fixed` bytes of static shared memory.  (What a launch
+// asks for decides how many CTAs fit an SM.)
 template <class Kernel>
-cudaError_t set_smem(Kernel* kern, size_t smem) {
-    if (smem > kMaxDynSmem) return cudaErrorInvalidValue;
+cudaError_t allow_smem(Kernel* kern, size_t smem, size_t fixed = 0) {
+    if (smem > kMaxDynSmem - fixed) return cudaErrorInvalidValue;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem));
+                                static_cast<int>(kMaxDynSmem - fixed));
 }
 
 template <class K>
@@ -201,8 +203,8 @@ cudaError_t launch_grid(K, const FwdParams& P, int n_jobs, cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(s, &cap);
     if (e != cudaSuccess) return e;
-    if (cap == cudaStreamCaptureStatusNone) {  // (set before a capture)
-        e = set_smem(kern, smem);
+    if (cap == cudaStreamCaptureStatusNone) {  // (allowed before a capture)
+        e = allow_smem(kern, smem);
         if (e != cudaSuccess) return e;
     }
     kern<<<grid, K::threads, smem, s>>>(P);
@@ -1296,9 +1298,7 @@ inline int adj_stage_cap(int ns, int minb, int eb) {
 template <bool AMP, int MINB, bool FIX>
 cudaError_t launch_adj(const psm::AdjParams& A, dim3 grid, dim3 block, size_t smem,
                        cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(psm::adj_kernel<AMP, MINB, FIX>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = allow_smem(psm::adj_kernel<AMP, MINB, FIX>, smem);
     if (e != cudaSuccess) return e;
     psm::adj_kernel<AMP, MINB, FIX><<<grid, block, smem, s>>>(A);
     return cudaGetLastError();
@@ -1923,13 +1923,17 @@ auto items_kernel() {
     return psm::fwd_items_kernel<K::AMP, K::KAHAN, K::NX, K::CAP, K::MINB>;
 }
 
-// Shared-memory attribute and persistent grid (resident CTAs on every SM) of the batch
+// Static shared memory of the persistent kernel (its tile and job) at most.
+constexpr size_t kBatchStaticSmem = 128;
+static_assert(sizeof(psm::BatchItem) + sizeof(Job) <= kBatchStaticSmem, "s_item, s_job");
+
+// Shared-memory limit and persistent grid (resident CTAs on every SM) of the batch
 // kernel K; done before a stream capture, so the graph holds only the launch.
 template <class K>
 cudaError_t prepare_persistent(K, psm_batch& b) {
     auto* kern = persistent_kernel<K>();
     const size_t smem = batch_smem<K>(b);
-    cudaError_t e = set_smem(kern, smem);
+    cudaError_t e = allow_smem(kern, smem, kBatchStaticSmem);
     if (e != cudaSuccess) return e;
     int per_sm = 0, n_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, K::threads, smem);
@@ -2018,11 +2022,11 @@ int batch_launch(psm_batch* b) {
             cudaGraphExecDestroy(b->exec);
             b->exec = nullptr;
         }
-        // the kernels' shared-memory attributes are set outside the capture
+        // the kernels' shared-memory limits are set outside the capture
         if (b->mode == PSM_BATCH_ONE_GRID)
             PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
                              using K = decltype(k);
-                             return set_smem(items_kernel<K>(), batch_smem<K>(*b));
+                             return allow_smem(items_kernel<K>(), batch_smem<K>(*b));
                          }));
         else if (b->mode == PSM_BATCH_PERSISTENT)
             PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
@@ -2032,7 +2036,7 @@ int batch_launch(psm_batch* b) {
             for (bool narrow : {false, true})
                 PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, narrow, [&](auto k) {
                                  using K = decltype(k);
-                                 return set_smem(grid_kernel<K>(), batch_smem<K>(*b));
+                                 return allow_smem(grid_kernel<K>(), batch_smem<K>(*b));
                              }));
         cudaGraph_t graph = nullptr;
         PSM_CUDA_TRY(c->st, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
