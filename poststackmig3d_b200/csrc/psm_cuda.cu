@@ -590,6 +590,14 @@ cudaError_t download(HostStaging& H, void* dst, const void* src, size_t bytes, c
     return cudaSuccess;
 }
 
+// The kernels' error word, zero from its allocation on: a call that returns an image reads it also
+// when no kernel has run.
+cudaError_t ensure_error_word(psm_ctx* c) {
+    if (c->err.p) return cudaSuccess;
+    const cudaError_t e = c->err.ensure(sizeof(int));
+    return e != cudaSuccess ? e : cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream);
+}
+
 int read_device_error(psm_ctx* c) {
     int h = 0;
     PSM_CUDA_TRY(c->st, cudaMemcpyAsync(&h, c->err.p, sizeof(int), cudaMemcpyDeviceToHost,
@@ -718,8 +726,8 @@ int psm_set_geometry(psm_ctx* c, const psm_geom* g, const int32_t* out_center) {
     PSM_CUDA_TRY(c->st, c->d_jobs_all.ensure(c->jobs_all.size() * sizeof(Job)));
     PSM_CUDA_TRY(c->st, c->il_pos.ensure(g->n_il * sizeof(int)));
     PSM_CUDA_TRY(c->st, c->t0.ensure(g->n_t * sizeof(float)));
-    PSM_CUDA_TRY(c->st, c->err.ensure(sizeof(int)));
-        std::vector<int> pos(g->n_il);
+    PSM_CUDA_TRY(c->st, ensure_error_word(c));
+    std::vector<int> pos(g->n_il);
     for (int i = 0; i < g->n_il; ++i) pos[i] = i;
     std::vector<float> t0(g->n_t);
     for (int i = 0; i < g->n_t; ++i)
@@ -2148,7 +2156,7 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
     if (!fits_staging(max_inl, max_nt, b->store == psm::kStoreF32 ? 8 : 4))
         return c->st.fail(PSM_ERR_UNSUPPORTED, "problems too large for one staging ring");
     cudaStream_t s = c->stream;
-    PSM_CUDA_TRY(c->st, c->err.ensure(sizeof(int)));
+    PSM_CUDA_TRY(c->st, ensure_error_word(c));
     for (BatchCube& q : b->cubes) {
         const size_t n = static_cast<size_t>(q.n_il) * q.n_xl * q.ns;
         PSM_CUDA_TRY(c->st, q.data.ensure(n * sizeof(float)));
