@@ -60,7 +60,11 @@ struct FwdStage {
 
 // Shared memory of a CTA: CAP samples a stage, folded windows of 8 bytes a sample.  A trace's
 // own raw samples are copied into the upper end of the memory that its folded window takes,
-// its mirror's into a buffer of their own.
+// its mirror's into a buffer of their own, one per stage.  Caller-made pairs (8 bytes a sample) have
+// one mirror buffer for all stages, so that as many CTAs fit an SM as with fp32 traces: the
+// producer waits for the folder to be done with it, which it is long before the consumers
+// release a stage.  (psm_forward_noalloc, 101 x 101 x 501 samples: 2.71 ms with a buffer per stage,
+// which leaves room for one CTA of the wide tiles, 2.04 ms so.)
 template <int NX, int CAP>
 struct FwdLayout {
     static_assert(NX % 2 == 0 && CAP % 8 == 0, "crossline pairs; 16-byte aligned windows");
@@ -74,8 +78,12 @@ struct FwdLayout {
     static constexpr unsigned kRing = (kBlk + 8 * 32 + 127) & ~127u;
     static constexpr unsigned kStageBytes = 8u * CAP;
     static constexpr unsigned kMirror = kRing + kStages * kStageBytes;
+    // bytes from one stage's mirror buffer to the next
+    static __host__ __device__ constexpr unsigned mirror_step(int store) {
+        return store == kStorePairs ? 0u : static_cast<unsigned>(CAP) * store_bytes(store);
+    }
     static __host__ __device__ constexpr unsigned rows(int store) {
-        return kMirror + kStages * static_cast<unsigned>(CAP) * store_bytes(store);
+        return kMirror + (store == kStorePairs ? 8u * CAP : kStages * mirror_step(store));
     }
     // row tables: running slot counts and dx^2
     static __host__ __device__ constexpr unsigned total(int store, int max_rows) {
@@ -548,7 +556,10 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             if (n > 0) {
                 const int stage = it % kStages;
                 const uint32_t par = ((it / kStages) & 1u) ^ 1u;
-                const int ok = lane == 0 ? mbar_wait(&empty[stage], par, P.err, P.wait_us) : 0;
+                int ok = lane == 0 ? mbar_wait(&empty[stage], par, P.err, P.wait_us) : 0;
+                if (lane == 0 && ok && store == kStorePairs && it > it_begin)  // the mirror buffer
+                    ok = mbar_wait(&ready[(it - 1) % kStages], ((it - 1) / kStages) & 1u, P.err,
+                                   P.wait_us);
                 if (!__shfl_sync(0xffffffffu, ok, 0)) {
                     alive = false;
                     break;
@@ -566,7 +577,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                     store == kStoreF32 ? L::kRing + stage * L::kStageBytes + 4u * (tot + off)
                                        : dst + (8u - rb) * copy;
                 const uint32_t dst_mir =
-                    L::kMirror + (static_cast<uint32_t>(stage) * CAP + off) * rb;
+                    L::kMirror + static_cast<uint32_t>(stage) * L::mirror_step(store) + off * rb;
                 const int slot = __popc(slots & ((1u << lane) - 1u));
                 if (mine) {
                     m.base[slot] = static_cast<int>(dst - 8u * ws - 0x58000000u);
