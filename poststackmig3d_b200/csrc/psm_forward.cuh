@@ -359,10 +359,11 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
     }
     // The producer's share of the wait: smallest and largest t0 of each block of 32 samples (lane
     // b holds block b), whatever their order (the per-inline call takes the caller's times).
-    // A sample has terms only with t0 > 0; every other counts as 0.
+    // A sample has terms only with t0 > 0; every other counts as 0.  (Not unrolled: 8.84 against
+    // 8.81 ms, 133 x 87 x 733 samples.)
     float t0min = 0.0f, t0max = 0.0f;
     if (warp == 0) {
-#pragma unroll
+#pragma unroll 1
         for (int b = 0; b < kTileT / 32; ++b) {
             const float t = __ldg(P.t0 + min(T0 + 32 * b + lane, P.n_t - 1));
             const int bits = t > 0.0f ? __float_as_int(t) : 0;
