@@ -241,10 +241,9 @@ __device__ __forceinline__ void adj_visit_fixed(unsigned char* sbase, float r2, 
 // the same address.  A lane's samples t, t + 1 touch at most the addresses l, l + 1, l + 2 with
 // l = floor(s(t)), and below the couple's r^2 bound `safe` (safe_reach) l grows from lane to
 // lane and from block to block, so the lanes' addresses l + k of one k are distinct: three
-// steps, k = 0, 1, 2, with a warp barrier between them.  Two blocks of 64 samples go together
-// (two independent chains of load, add and store).  A lane whose second sample lands beyond
+// steps, k = 0, 1, 2, with a warp barrier between them.  N blocks of 64 samples go together
+// (independent chains of load, add and store).  A lane whose second sample lands beyond
 // l + 1 (rounding at ds/dt0 = 1, a falling Vrms) sends its blocks through the atomics.
-// N blocks of 64 samples go together (independent chains of load, add and store).
 // floor(s) of a passing term is n_t - 1 at most (a fast s that rounds up): its share beyond the
 // record falls on the window's sample n_t, which the flush drops.
 // False when it left the blocks to the atomics.
@@ -458,7 +457,6 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
         // are two samples apart, so their trace samples (ds/dt0 = t0 / t >= cos(aperture) inside
         // the aperture of a constant Vrms, 0.7 at 45 deg) fall on different window addresses;
         // couples of blocks span 128 consecutive samples
-        bool sane = true;  // every sample of the record has a Vrms
 #pragma unroll
         for (int p = 0; p < kJ / 2; ++p) {
             float t2[2], f4[2], bj[2], mk[2];
@@ -470,7 +468,6 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     v = __ldg(vp + t);
                     t0v = __ldg(P.t0 + t);
                     mv = __ldg(mp + t);
-                    sane = sane && v >= 1e-5f;
                 }
                 const PointConst pc = point_const(v, t0v, P.tan2);
                 const float b = pass_bound<false>(pc, P.inv_dt, P.ntm1f);
@@ -484,7 +481,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     // neighbour's, their shares are zero)
                     const bool in = xvalid && t < P.n_t;
                     t2[k] = in ? fmaxf(pc.t0sq * P.idt2, 0.25f) : kBeyond;
-                    f4[k] = in && v >= 1e-5f ? pc.f4 * P.idt2 : 0.0f;
+                    f4[k] = !in ? 0.0f : v >= 1e-5f ? pc.f4 * P.idt2 : -1.0f;
                 }
                 if (b >= 0.0f) {
                     t2[k] = pc.t0sq * P.idt2;
@@ -496,6 +493,21 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     t0min = fminf(t0min, t0v);
                     t0max = fmaxf(t0max, t0v);
                 }
+            }
+            if (!FIX && __any_sync(0xffffffffu, fminf(f4[0], f4[1]) < 0.0f)) {
+                // a sample without a Vrms takes that of the lane's other sample, else of the
+                // nearest lane below that has one, else of the first lane that has one: the
+                // lanes' order, and with it `safe`, holds across it (101 x 101 x 501 samples, one
+                // in 97 without a Vrms: 8.06 ms with the warp's blocks through the atomics, 5.35
+                // so, 6.65 with atomics everywhere in 4 CTAs per SM)
+                const float own = fmaxf(f4[0], f4[1]);
+                const unsigned have = __ballot_sync(0xffffffffu, own > 0.0f);
+                const unsigned below = have & ((1u << lane) - 1u);
+                const float other =
+                    __shfl_sync(0xffffffffu, own, below ? 31 - __clz(below) : __ffs(have) - 1);
+                const float f = own > 0.0f ? own : have ? other : 0.0f;
+                if (f4[0] < 0.0f) f4[0] = f;
+                if (f4[1] < 0.0f) f4[1] = f;
             }
             T2[p] = make_float2(t2[0], t2[1]);
             F4[p] = make_float2(f4[0], f4[1]);
@@ -553,7 +565,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     if ((lane < 31 || k == 0) && top >= 0.0f && t2.x < kBeyond)
                         r = fminf(r, safe_reach(t2.x, f4.x, tn, fn, top));
                 }
-                safe[h] = __all_sync(0xffffffffu, sane) ? warp_min(r) : -1.0f;
+                safe[h] = warp_min(r);
             }
         }
         vmin = warp_min(vmin);
