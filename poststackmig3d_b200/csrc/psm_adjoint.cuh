@@ -360,6 +360,23 @@ __device__ __forceinline__ void adj_visit(unsigned char* sbase, float r2, uint32
     }
 }
 
+// One slot for one couple of blocks with atomics; full: every lane of the couple passes.
+template <bool AMP>
+__device__ __forceinline__ void adj_visit_atomic(unsigned char* sbase, float r2, uint32_t base,
+                                                 float smax, bool full, const float2* T2,
+                                                 const float2* F4, const float2* BB,
+                                                 const float2* MK) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        if (full)
+            adj_term2<AMP, false>(sbase, r2, base, smax, T2[j].x, F4[j].x, BB[j].x, MK[j].x,
+                                  T2[j].y, F4[j].y, BB[j].y, MK[j].y);
+        else
+            adj_term2<AMP, true>(sbase, r2, base, smax, T2[j].x, F4[j].x, BB[j].x, MK[j].x,
+                                 T2[j].y, F4[j].y, BB[j].y, MK[j].y);
+    }
+}
+
 // Add the windows of one released stage into the data cube (one bulk reduction per window and
 // trace, lanes in parallel; a pair's window goes to both of its traces) and wait until they
 // have read shared memory.  FIX: the stage's 64-bit integer sums are first turned into FP64
@@ -416,11 +433,13 @@ __device__ __forceinline__ void adj_flush(const AdjParams& A, const AdjMeta& m,
     __syncwarp();
 }
 
-// MINB: CTAs per SM the kernel is built for (the host gives 3-CTA launches 32 KB stages): more
-// warps hide the latency of the shared-memory additions.
+// MINB: CTAs per SM the kernel is built for (the host gives 3-CTA launches 32 KB stages, 4-CTA
+// launches 20 KB): more warps hide the latency of the shared-memory additions.
 // FIX: 64-bit fixed-point window sums (atomics) and an FP64 data cube (A.data64); else fp32 sums
 // and an fp32 data cube (A.data).
-template <bool AMP, int MINB = 2, bool FIX = false>
+// OWN: a warp owns the window it adds into; else fp32 sums with atomics, for steep apertures, in
+// which most terms lie beyond `safe` (kSteepTan2).
+template <bool AMP, int MINB = 2, bool FIX = false, bool OWN = !FIX>
 __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjParams A) {
     constexpr int EB = FIX ? 8 : 4;           // bytes of a window sample
     constexpr uint32_t MAGIC = FIX ? kMagic8 : kMagic4;
@@ -473,7 +492,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                 const float b = pass_bound<false>(pc, P.inv_dt, P.ntm1f);
                 bj[k] = b;
                 mk[k] = 0.0f;
-                if (FIX) {
+                if (!OWN) {
                     t2[k] = 1.0f;
                     f4[k] = 0.0f;
                 } else {
@@ -494,7 +513,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                     t0max = fmaxf(t0max, t0v);
                 }
             }
-            if (!FIX && __any_sync(0xffffffffu, fminf(f4[0], f4[1]) < 0.0f)) {
+            if (OWN && __any_sync(0xffffffffu, fminf(f4[0], f4[1]) < 0.0f)) {
                 // a sample without a Vrms takes that of the lane's other sample, else of the
                 // nearest lane below that has one, else of the first lane that has one: the
                 // lanes' order, and with it `safe`, holds across it (101 x 101 x 501 samples, one
@@ -521,7 +540,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
             gmin[h] = warp_min(fminf(fminf(u.x, u.y), fminf(w.x, w.y)));
             warpmax = fmaxf(warpmax, gmax[h]);
             safe[h] = -1.0f;
-            if (!FIX && gmax[h] >= 0.0f) {
+            if (OWN && gmax[h] >= 0.0f) {
                 // each gap between two lanes' first samples (the last lane's next is the
                 // couple's second block's first) has to be good up to the largest r^2 at which
                 // lanes on both sides of it have terms
@@ -797,7 +816,7 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
         const int stage = it % kStages;
         const uint32_t par = (it / kStages) & 1u;
         bool ok = mbar_wait(&full[stage], par, P.err, P.wait_us);
-        if (!FIX) ok = consumers_agree(ok);  // (the steps' barriers need every warp)
+        if (OWN) ok = consumers_agree(ok);  // (the steps' barriers need every warp)
         if (!ok) break;
         const AdjMeta& m = meta[stage];
         const int cnt = m.count;
@@ -808,6 +827,21 @@ __global__ void __launch_bounds__(32 * (kTX + 1), MINB) adj_kernel(const AdjPara
                 if (r2 > warpmax) continue;
                 adj_visit_fixed<AMP>(smem_raw, r2, static_cast<uint32_t>(m.m[g]), P.ntm1m, gmax,
                                      gmin, T2, F4, BB, MK);
+            }
+            __syncwarp();
+        } else if constexpr (!OWN) {
+            const float* r2w = m.r2[warp - 1];
+            const float own = lane < cnt ? r2w[lane] : 3.0e38f;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const unsigned full2 = __ballot_sync(0xffffffffu, own <= gmin[h]);
+                for (unsigned todo = __ballot_sync(0xffffffffu, own <= gmax[h]); todo;
+                     todo &= todo - 1) {
+                    const int g = __ffs(todo) - 1;
+                    adj_visit_atomic<AMP>(smem_raw, r2w[g], static_cast<uint32_t>(m.m[g]),
+                                          P.ntm1m, (full2 >> g) & 1u, T2 + 2 * h, F4 + 2 * h,
+                                          BB + 2 * h, MK + 2 * h);
+                }
             }
             __syncwarp();
         } else {

@@ -1297,18 +1297,27 @@ int psm_forward_host(psm_ctx* c, const float* traces, const float* vrms, float* 
 
 namespace {
 
+// From this tan^2 of the aperture on (just below 60 degrees), fp32 sums go through atomics in 4 CTAs
+// per SM: where Vrms rises, most terms lie where lanes' addresses meet, and the 3-CTA kernel would
+// send them through atomics too.  61 x 61 x 501 samples, with owned windows and so, ms:
+//   Vrms           55 deg        60 deg        65 deg        70 deg
+//   2000           2.06, 2.84    2.92, 3.27    3.66, 3.84    4.41, 4.26
+//   1800 to 2600   3.34, 3.57    4.19, 4.18    4.97, 4.79    6.60, 5.73
+//   1500 to 3500   4.99, 5.01    7.72, 6.94    10.20, 8.62   11.65, 9.29
+constexpr float kSteepTan2 = 2.9f;
+
 // Samples per adjoint ring stage: 48 KB stages (32 KB for 3 CTAs per SM) of 4-byte fp32 sums
 // or 8-byte fixed-point sums, and at least one whole trace.
 inline int adj_stage_cap(int ns, int minb, int eb) {
-    return std::max((minb == 3 ? 32768 : 49152) / eb, ns);
+    return std::max((minb == 4 ? 20480 : minb == 3 ? 32768 : 49152) / eb, ns);
 }
 
-template <bool AMP, int MINB, bool FIX>
+template <bool AMP, int MINB, bool FIX, bool OWN = !FIX>
 cudaError_t launch_adj(const psm::AdjParams& A, dim3 grid, dim3 block, size_t smem,
                        cudaStream_t s) {
-    cudaError_t e = allow_smem(psm::adj_kernel<AMP, MINB, FIX>, smem);
+    cudaError_t e = allow_smem(psm::adj_kernel<AMP, MINB, FIX, OWN>, smem);
     if (e != cudaSuccess) return e;
-    psm::adj_kernel<AMP, MINB, FIX><<<grid, block, smem, s>>>(A);
+    psm::adj_kernel<AMP, MINB, FIX, OWN><<<grid, block, smem, s>>>(A);
     return cudaGetLastError();
 }
 
@@ -1344,11 +1353,17 @@ int adjoint_dev(psm_ctx* c, const float* d_rows, float* d_out) {
         PSM_CUDA_TRY(c->st, cudaMemsetAsync(d_out, 0, n_data * sizeof(float), c->stream));
     }
     const int eb = fix ? 8 : 4;
-    // 3 CTAs per SM when their 32 KB stages and the inline tables fit a third of the SM, else 2
-    A.F.stage_cap = adj_stage_cap(c->ns, 3, eb);
+    // 3 CTAs per SM when their 32 KB stages and the inline tables fit a third of the SM, else 2;
+    // steep apertures (kSteepTan2): 4 when their 20 KB stages fit
+    A.F.stage_cap = adj_stage_cap(c->ns, 4, eb);
     size_t smem = psm::adj_layout(A.F.max_inl, A.F.stage_cap, eb).total;
-    const bool o3 = smem <= 75 * 1024;
-    if (!o3) {
+    const bool o4 = !fix && c->g.tan2_theta >= kSteepTan2 && smem <= 56 * 1024;
+    if (!o4) {
+        A.F.stage_cap = adj_stage_cap(c->ns, 3, eb);
+        smem = psm::adj_layout(A.F.max_inl, A.F.stage_cap, eb).total;
+    }
+    const bool o3 = !o4 && smem <= 75 * 1024;
+    if (!o3 && !o4) {
         A.F.stage_cap = adj_stage_cap(c->ns, 2, eb);
         smem = psm::adj_layout(A.F.max_inl, A.F.stage_cap, eb).total;
     }
@@ -1365,6 +1380,9 @@ int adjoint_dev(psm_ctx* c, const float* d_rows, float* d_out) {
                       : launch_adj<false, 3, true>(A, grid, block, smem, c->stream))
                : (amp ? launch_adj<true, 2, true>(A, grid, block, smem, c->stream)
                       : launch_adj<false, 2, true>(A, grid, block, smem, c->stream));
+    else if (o4)
+        e = amp ? launch_adj<true, 4, false, false>(A, grid, block, smem, c->stream)
+                : launch_adj<false, 4, false, false>(A, grid, block, smem, c->stream);
     else
         e = o3 ? (amp ? launch_adj<true, 3, false>(A, grid, block, smem, c->stream)
                       : launch_adj<false, 3, false>(A, grid, block, smem, c->stream))
