@@ -267,15 +267,12 @@ __device__ __forceinline__ bool range_ok(float r2, float f4, float t0sq, float i
     return __fmul_rn(__fsqrt_rn(__fmaf_rn(f4, r2, t0sq)), inv_dt) < ntm1f;
 }
 
-// GALLOP: start from an estimate of the boundary (fewer evaluations; the adjoint keeps the
-// plain bisection, whose smaller code spills less in its 4-CTA build).
-template <bool GALLOP = true>
 __device__ __forceinline__ float pass_bound(const PointConst& p, float inv_dt, float ntm1f) {
     if (!p.valid || !(p.md2 >= 0.0f)) return -1.0f;
     if (range_ok(p.md2, p.f4, p.t0sq, inv_dt, ntm1f)) return p.md2;
     if (!range_ok(0.0f, p.f4, p.t0sq, inv_dt, ntm1f)) return -1.0f;
     unsigned lo = 0u, hi = __float_as_uint(p.md2);  // ok(lo), !ok(hi)
-    if (GALLOP && hi - lo > 1u) {
+    if (hi - lo > 1u) {
         // Gallop out from the boundary of the unrounded test, f4 r2 + t0^2 =
         // ((n_t - 1) / inv_dt)^2, to a bracket of doubling width; the bisection below then
         // closes it.  The test is monotone in r2, so any bracket gives the same bound as a
