@@ -154,10 +154,14 @@ template <bool AMP, bool KAHAN, bool ORDERED>
 using NarrowTag = KernelTag<AMP, KAHAN, ORDERED, kNarrowNX, 2432, 3>;
 
 // Narrow tiles for a problem whose wide tiles do not fill the SMs (launches of a few jobs of a
-// larger problem keep the problem's tiles, so that their images are the same bit for bit).
+// larger problem keep the problem's tiles, so that their images are the same bit for bit), and for
+// one with no more crosslines than a narrow tile has, which leave most warps of a wide tile
+// without work (wide, narrow: 1001 x 1 x 1001 samples 0.502, 0.347 ms, 1001 x 4 x 1001 1.437,
+// 1.072, 201 x 5 x 501 0.160, 0.171).
 inline bool few_tiles(int64_t n_jobs, int n_ox, int n_t) {
-    return n_jobs * ((n_ox + kWideNX - 1) / kWideNX) * ((n_t + psm::kTileT - 1) / psm::kTileT) <
-           148;
+    return n_ox <= kNarrowNX ||
+           n_jobs * ((n_ox + kWideNX - 1) / kWideNX) * ((n_t + psm::kTileT - 1) / psm::kTileT) <
+               148;
 }
 // Whether `variant` runs narrow tiles (`few`: the problem's own choice, taken by the default).
 inline bool narrow_tiles(int variant, int store, bool kahan, bool few) {

@@ -1,0 +1,44 @@
+"""The tiles that the default variant takes: which of the two kernels a problem runs, told by its
+image bit for bit (the two add an output sample's terms in different orders)."""
+import numpy as np
+import pytest
+
+from poststackmig3d_b200 import Migrator
+from poststackmig3d_b200 import synth as S
+
+from helpers import geometry_for
+
+pytestmark = pytest.mark.gpu
+
+DEFAULT, WIDE, NARROW = 0, 11, 12
+
+
+def _workload(n_il, n_xl, n_t, pad_xl=0, seed=5):
+    return S.random_workload(seed, n_il, n_xl, n_t, vel_kind="lateral", angle=50.0, d_il=14.0,
+                             d_xl=11.0, pad_xl=pad_xl)
+
+
+def _context(m, W, g):
+    m.set_geometry(g)
+    m.set_traces(W.data)
+    m.set_vrms(W.vrms_cube())
+
+
+def _images(W, g):
+    with Migrator(0) as m:
+        _context(m, W, g)
+        out = {}
+        for v in (DEFAULT, WIDE, NARROW):
+            m.set_variant(v)
+            out[v] = m.forward()
+    assert not np.array_equal(out[WIDE], out[NARROW])  # the case tells them apart
+    return out
+
+
+@pytest.mark.parametrize("n_il,n_xl,n_t,pad_xl,narrow", [
+    (90, 2, 260, 1, True), (90, 3, 260, 1, False),  # 4 and 5 output crosslines
+    (73, 5, 260, 0, True), (74, 5, 260, 0, False)])  # 146 and 148 wide tiles
+def test_default_tiles(n_il, n_xl, n_t, pad_xl, narrow):
+    W = _workload(n_il, n_xl, n_t, pad_xl)
+    img = _images(W, geometry_for(W))
+    assert np.array_equal(img[DEFAULT], img[NARROW if narrow else WIDE])
