@@ -269,6 +269,9 @@ typedef enum {
     PSM_FWD_N_VARIANTS = 14
 } psm_fwd_variant;
 int psm_set_variant(psm_ctx *ctx, int variant);
+/* The variant that a forward runs: for PSM_FWD_DEFAULT the one it stands for on the current
+ * geometry, for an id that 16-bit storage or compensated summation does not know the one it
+ * stands for there. */
 int psm_get_variant(psm_ctx *ctx, int *variant);
 /* Time one forward launch of each kernel on the resident cube (CUDA events on the ctx
  * stream), keep the fastest for this ctx.  ms[PSM_FWD_N_VARIANTS] (may be NULL) receives every

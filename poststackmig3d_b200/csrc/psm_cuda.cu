@@ -132,6 +132,7 @@ inline int effective_variant(int variant, int store, bool kahan) {
     const bool j16 = variant == PSM_FWD_PACKED_G4_J16 || variant == PSM_FWD_SCALAR_G4_J16;
     if (!kahan && j16) return PSM_FWD_PACKED_G4_J16;
     if (variant == PSM_FWD_PAIRS_O3 || variant == PSM_FWD_PAIRS) return variant;
+    if (variant == PSM_FWD_PAIRS_J4_O4) return PSM_FWD_PAIRS;  // (narrow tiles too)
     return variant == PSM_FWD_PACKED_G4_O3 || variant == PSM_FWD_SCALAR_G4_O3
                ? PSM_FWD_PACKED_G4_O3
                : PSM_FWD_PACKED_G4;
@@ -168,6 +169,11 @@ inline bool narrow_tiles(int variant, int store, bool kahan, bool few) {
     if (variant == PSM_FWD_DEFAULT) return few;
     const int v = effective_variant(variant, store, kahan);
     return v == PSM_FWD_PAIRS || v == PSM_FWD_PAIRS_J4_O4;
+}
+// The id that the getters report: the default's is that of the tiles it takes.
+inline int reported_variant(int variant, int store, bool kahan, bool few) {
+    if (variant == PSM_FWD_DEFAULT) return few ? PSM_FWD_PAIRS : kDefaultVariant;
+    return effective_variant(variant, store, kahan);
 }
 
 // Calls f(KernelTag<...>{}) for the kernel that (amp, kahan, narrow) names.
@@ -1027,7 +1033,7 @@ int psm_set_variant(psm_ctx* c, int variant) {
 
 int psm_get_variant(psm_ctx* c, int* variant) {
     if (!c || !variant) return PSM_ERR_ARG;
-    *variant = effective_variant(c->variant, c->store, c->g.compensated != 0);
+    *variant = reported_variant(c->variant, c->store, c->g.compensated != 0, c->few);
     return PSM_OK;
 }
 
@@ -2337,7 +2343,7 @@ int psm_batch_set_variant(psm_batch* b, int variant) {
 
 int psm_batch_get_variant(psm_batch* b, int* variant) {
     if (!b || !variant) return PSM_ERR_ARG;
-    *variant = effective_variant(b->variant, b->store, b->kahan);
+    *variant = reported_variant(b->variant, b->store, b->kahan, b->few);
     return PSM_OK;
 }
 

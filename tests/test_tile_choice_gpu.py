@@ -1,5 +1,7 @@
 """The tiles that the default variant takes: which of the two kernels a problem runs, told by its
 image bit for bit (the two add an output sample's terms in different orders)."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -42,3 +44,24 @@ def test_default_tiles(n_il, n_xl, n_t, pad_xl, narrow):
     W = _workload(n_il, n_xl, n_t, pad_xl)
     img = _images(W, geometry_for(W))
     assert np.array_equal(img[DEFAULT], img[NARROW if narrow else WIDE])
+
+
+@pytest.mark.parametrize("n_il,narrow", [(73, True), (74, False)])
+@pytest.mark.parametrize("precision,compensated", [("f32", False), ("f32", True), ("bf16", False)])
+def test_reported_variant_is_the_one_that_runs(n_il, narrow, precision, compensated):
+    """The default's id is that of its tiles, and setting it gives the same image; id 13 runs the
+    narrow tiles with every storage and sum."""
+    W = _workload(n_il, 5, 260)
+    g = dataclasses.replace(geometry_for(W), precision=precision, compensated=compensated)
+    with Migrator(0) as m:
+        _context(m, W, g)
+        ref = m.forward()
+        v = m.variant()
+        assert v == (NARROW if narrow else WIDE)
+        m.set_variant(v)
+        assert np.array_equal(m.forward(), ref)
+        m.set_variant(NARROW)
+        img = m.forward()
+        m.set_variant(13)
+        assert np.array_equal(m.forward(), img)
+        assert m.variant() in (NARROW, 13)
