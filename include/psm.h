@@ -31,6 +31,9 @@ typedef enum {
 
 typedef enum { PSM_F32 = 0, PSM_BF16 = 1, PSM_F16 = 2 } psm_precision;
 
+/* Forward-kernel tiles of a problem under PSM_FWD_DEFAULT (psm_fwd_variant). */
+typedef enum { PSM_TILES_AUTO = 0, PSM_TILES_WIDE = 1, PSM_TILES_NARROW = 2 } psm_tiles;
+
 /* Geometry and migration parameters of a resident cube.  The values are the ones the
  * reference driver derives (src/main.cpp:124-217):
  *   n_il, n_xl, n_t   real input grid (sorted unique inline / crossline labels, samples)
@@ -57,6 +60,10 @@ typedef enum { PSM_F32 = 0, PSM_BF16 = 1, PSM_F16 = 2 } psm_precision;
  *                     OpenMP build computes (its per-sample caches, :60-72, are not reset for
  *                     crosslines with v = 0, and its nested crossline loop runs on one
  *                     thread, src/main.cpp:255); Vrms is taken to be positive.
+ *   tiles             psm_tiles: the tiles that PSM_FWD_DEFAULT takes, which set the order of
+ *                     an output sample's sum.  PSM_TILES_AUTO (0, and any value that is not a
+ *                     psm_tiles): by the problem's size.  psm_slab_geometry sets the whole
+ *                     problem's choice.
  */
 typedef struct {
     int32_t n_il, n_xl, n_t;
@@ -71,6 +78,7 @@ typedef struct {
     double dt_seconds;
     int32_t compensated;
     int32_t compat_omp_pad;
+    int32_t tiles;
 } psm_geom;
 
 typedef struct psm_ctx psm_ctx;
@@ -130,8 +138,8 @@ int psm_stream(psm_ctx *ctx, void **stream);
  * file (prepareInputBufferWithPadding, src/migration_kernel.cpp:385-468).  A slab is output
  * inlines [o0, o1) and the input inlines [i0, i1) their buffers read (each output inline o
  * reads [c - m_il - pad_il, c + m_il + 1 + pad_il) around its centre c, clamped to the cube,
- * migration_kernel.cpp:404-409); migrating the slab on its own gives exactly those rows of the
- * whole image. */
+ * migration_kernel.cpp:404-409); migrating the slab on its own, with the geometry that
+ * psm_slab_geometry gives, gives exactly those rows of the whole image. */
 typedef struct {
     int32_t o0, o1; /* output inlines */
     int32_t i0, i1; /* input inlines */

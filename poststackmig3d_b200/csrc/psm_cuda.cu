@@ -164,6 +164,13 @@ inline bool few_tiles(int64_t n_jobs, int n_ox, int n_t) {
            n_jobs * ((n_ox + kWideNX - 1) / kWideNX) * ((n_t + psm::kTileT - 1) / psm::kTileT) <
                148;
 }
+// Whether a problem takes narrow tiles by default: as its geometry says (a slab's, for the whole
+// problem), else by its own size.
+inline bool default_narrow(const psm_geom& g, int64_t n_jobs) {
+    if (g.tiles == PSM_TILES_WIDE || g.tiles == PSM_TILES_NARROW)
+        return g.tiles == PSM_TILES_NARROW;
+    return few_tiles(n_jobs, g.n_ox, g.n_t);
+}
 // Whether `variant` runs narrow tiles (`few`: the problem's own choice, taken by the default).
 inline bool narrow_tiles(int variant, int store, bool kahan, bool few) {
     if (variant == PSM_FWD_DEFAULT) return few;
@@ -388,7 +395,7 @@ struct psm_ctx {
     DevBuf data, vrms, image, d_jobs, d_jobs_all, il_pos, t0, err, count;
     int tail_nt = 0;        // samples per trace up to which `data` is written, and the bytes of
     size_t tail_bytes = 0;  // it whose rows' tails are known to be zero for that length
-    bool few = false;       // narrow tiles by default (few_tiles)
+    bool few = false;       // narrow tiles by default (default_narrow)
     // 16-bit storage: samples [n_il][n_xl][ns] and one scale per trace
     DevBuf words, scales;
     // adjoint: rows of each job (fold of duplicated output rows), image upload, job images
@@ -713,7 +720,7 @@ int psm_set_geometry(psm_ctx* c, const psm_geom* g, const int32_t* out_center) {
     c->jobs.swap(jobs);
     c->jobs_all.swap(jobs_all);
     c->copies.swap(copies);
-    c->few = few_tiles(static_cast<int64_t>(c->jobs.size()), g->n_ox, g->n_t);
+    c->few = default_narrow(*g, static_cast<int64_t>(c->jobs.size()));
     const size_t n_tr = static_cast<size_t>(g->n_il) * g->n_xl;
     const size_t cube = n_tr * ns * sizeof(float);
     if (cube > c->data.bytes) c->tail_bytes = 0;  // reallocated below
@@ -1701,7 +1708,16 @@ int psm_slab_geometry(const psm_geom* g, const int32_t* out_center, const psm_sl
     psm_slab need{s->o0, s->o1, 0, 0};
     slab_range(*g, out_center, &need);
     if (s->i0 < 0 || s->i1 > g->n_il || s->i0 > need.i0 || s->i1 < need.i1) return PSM_ERR_ARG;
+    // the whole problem's tiles, so that the slab's image is its rows bit for bit
+    std::vector<char> seen(g->n_il, 0);
+    int64_t n_jobs = 0;
+    for (int o = 0; o < g->n_oi; ++o) {
+        char& c = seen[slab_center(*g, out_center, o)];
+        n_jobs += !c;
+        c = 1;
+    }
     *local = *g;
+    local->tiles = default_narrow(*g, n_jobs) ? PSM_TILES_NARROW : PSM_TILES_WIDE;
     local->n_il = s->i1 - s->i0;
     local->n_oi = s->o1 - s->o0;
     for (int o = s->o0; o < s->o1; ++o)
@@ -1747,10 +1763,6 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
             keep[k] = std::min(slabs[k - 1].i1, sl.i1) - sl.i0;
         if (k > 0 && keep[k] > 0) max_fresh = std::max(max_fresh, (sl.i1 - sl.i0) - keep[k]);
     }
-    std::vector<Job> all, all_rows;
-    std::vector<std::pair<int, int>> reps;
-    plan_jobs(*g, out_center, all, all_rows, reps);
-    const bool few = few_tiles(static_cast<int64_t>(all.size()), g->n_ox, g->n_t);
     // size the device buffers for the widest slab once, so that none regrows
     if (n > 1 && (rc = psm_set_geometry(c, &loc[wide], lcs[wide].data()))) return rc;
     for (cudaStream_t* t : {&c->copy_stream, &c->d2h_stream})
@@ -1797,7 +1809,6 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
         const bool had = k > 0 && c->have_traces && c->have_vrms;
         // (waits for slab k - 1's kernel: psm_set_geometry synchronises the stream)
         if ((rc = psm_set_geometry(c, &loc[k], lcs[k].data()))) return rc;
-        c->few = few;  // the tiles of the whole problem: slab images are its rows bit for bit
         bool same_bufs = true;
         for (int i = 0; i < 4; ++i)
             if ((i == 0 || i == 3 || c->store != psm::kStoreF32) && bufs[i]->bytes != sizes[i])
@@ -1922,7 +1933,7 @@ struct psm_batch {
     int variant = PSM_FWD_DEFAULT;
     int mode = PSM_BATCH_PERSISTENT;
     int max_rows = 1;
-    bool few = true;  // every problem takes narrow tiles by itself (few_tiles)
+    bool few = true;  // every problem takes narrow tiles by itself (default_narrow)
     int grid = 1;  // persistent CTAs
     int order = PSM_ORDER_DEPTH_FIRST;
     // tile lists [wide / narrow tiles][order]
@@ -2005,8 +2016,7 @@ bool batch_narrow(const psm_batch& b) {
 }
 bool problem_narrow(const psm_batch& b, const BatchProblem& p) {
     return narrow_tiles(b.variant, b.store, b.kahan,
-                        few_tiles(static_cast<int64_t>(p.jobs.size()), p.src.geom.n_ox,
-                                  p.src.geom.n_t));
+                        default_narrow(p.src.geom, static_cast<int64_t>(p.jobs.size())));
 }
 
 // Repeated output rows of every problem (padded output inlines, main.cpp:268-285).
@@ -2179,7 +2189,7 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
         max_inl = std::max(max_inl, max_inline_window(p.jobs_all));
         max_nt = std::max(max_nt, g.n_t);
         b->max_rows = std::max(b->max_rows, max_list_rows(p.jobs_all));
-        b->few = b->few && few_tiles(static_cast<int64_t>(p.jobs.size()), g.n_ox, g.n_t);
+        b->few = b->few && default_narrow(g, static_cast<int64_t>(p.jobs.size()));
     }
     if (!fits_staging(max_inl, max_nt, b->store == psm::kStoreF32 ? 8 : 4))
         return c->st.fail(PSM_ERR_UNSUPPORTED, "problems too large for one staging ring");
@@ -2756,7 +2766,7 @@ extern "C" int psm_forward_noalloc(const psm_geom* g, const int32_t* out_center,
     P.il_pos = reinterpret_cast<const int*>(scratch + kNoallocPos);
     P.t0 = reinterpret_cast<const float*>(scratch + kNoallocT0);
     P.err = reinterpret_cast<int*>(scratch + kNoallocErr);
-    PSM_NA_TRY(launch_fwd(P, n_jobs, g->amp_correction != 0, few_tiles(n_jobs, g->n_ox, g->n_t), s));
+    PSM_NA_TRY(launch_fwd(P, n_jobs, g->amp_correction != 0, default_narrow(*g, n_jobs), s));
     const size_t row = static_cast<size_t>(g->n_ox) * g->n_t;
     for (int k = 0; k < n_dup; ++k)
         PSM_NA_TRY(cudaMemcpyAsync(d_image + dup_dst[k] * row, d_image + dup_src[k] * row,

@@ -110,6 +110,7 @@ class Geometry:
     precision: str = "f32"
     compensated: bool = False
     compat_omp_pad: bool = False  # trailing padded crosslines as the reference's OpenMP build
+    tiles: int = 0  # psm_tiles: 0 by the problem's size; a slab's are the whole problem's
 
     @property
     def dt(self) -> float:
@@ -125,7 +126,7 @@ class Geometry:
                        self.n_ox, self.m_il, int(bool(self.amp)), PRECISIONS[self.precision],
                        np.float32(self.dt_seconds), self.d_il, self.d_xl, self.tan2,
                        self.dt_seconds, int(bool(self.compensated)),
-                       int(bool(self.compat_omp_pad)))
+                       int(bool(self.compat_omp_pad)), int(self.tiles))
 
 
 def plan_geometry(n_il: int, n_xl: int, n_t: int, dt_seconds: float, d_il: float,
@@ -194,7 +195,8 @@ def slab_geometry(g: Geometry, slab: Slab) -> Geometry:
     check(_lib.cuda().psm_slab_geometry(ctypes.byref(gc), oc.ctypes.data, ctypes.byref(s),
                                         ctypes.byref(loc), lc.ctypes.data),
           lambda: "psm_slab_geometry")
-    return dataclasses.replace(g, n_il=loc.n_il, n_oi=loc.n_oi, out_center=lc[:loc.n_oi])
+    return dataclasses.replace(g, n_il=loc.n_il, n_oi=loc.n_oi, out_center=lc[:loc.n_oi],
+                               tiles=loc.tiles)
 
 
 def estimate_max_velocity(vrms: np.ndarray) -> float:

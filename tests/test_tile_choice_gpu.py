@@ -7,6 +7,7 @@ import pytest
 
 from poststackmig3d_b200 import Migrator
 from poststackmig3d_b200 import synth as S
+from poststackmig3d_b200.shard import migrate_shard
 
 from helpers import geometry_for
 
@@ -65,3 +66,18 @@ def test_reported_variant_is_the_one_that_runs(n_il, narrow, precision, compensa
         m.set_variant(13)
         assert np.array_equal(m.forward(), img)
         assert m.variant() in (NARROW, 13)
+
+
+@pytest.mark.parametrize("precision", ["f32", "f16"])
+def test_shards_are_the_whole_image(precision):
+    """A rank's slab has few tiles of its own and takes the whole problem's: its rows are the whole
+    image's bit for bit."""
+    W = _workload(75, 5, 260)
+    g = dataclasses.replace(geometry_for(W), precision=precision)
+    with Migrator(0) as m:
+        _context(m, W, g)
+        whole = m.forward()
+        assert m.variant() == WIDE
+    for world in (2, 5):
+        rows = [migrate_shard(g, W.data, W.vrms_cube(), r, world)[1] for r in range(world)]
+        assert np.array_equal(np.concatenate(rows), whole)
