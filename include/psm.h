@@ -296,7 +296,9 @@ int psm_count_terms_rows(psm_ctx *ctx, int64_t *per_row);
 /* ---- Batched migration: several problems (velocity-scan panels over one cube, uneven
  * sub-volumes with their own Vrms) in ONE persistent launch, replayed as a CUDA graph.  No
  * counterpart in the reference, which migrates one cube with one velocity field per run
- * (src/main.cpp:291-361); each problem is exactly that run's operator. */
+ * (src/main.cpp:291-361); each problem is exactly that run's operator.  With PSM_FWD_DEFAULT a
+ * problem takes the tiles that it takes by itself, in every mode, and its image is that of a
+ * migration by itself bit for bit; a batch of both tiles then has a launch of each. */
 typedef enum {
     PSM_VRMS_CUBE = 0,     /* vrms [n_il][n_xl][n_t], as psm_set_vrms */
     PSM_VRMS_TRACE = 1,    /* vrms [n_t]: one Vrms(t) for every output point */

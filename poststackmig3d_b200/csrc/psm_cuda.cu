@@ -1916,6 +1916,7 @@ struct BatchCube {
 struct BatchProblem {
     psm_problem src{};
     int cube = 0;
+    bool few = false;  // narrow tiles by default (default_narrow)
     std::vector<Job> jobs, jobs_all;
     std::vector<std::pair<int, int>> copies;
     DevBuf vrms, image, d_jobs, d_jobs_all, t0;
@@ -1933,12 +1934,12 @@ struct psm_batch {
     int variant = PSM_FWD_DEFAULT;
     int mode = PSM_BATCH_PERSISTENT;
     int max_rows = 1;
-    bool few = true;  // every problem takes narrow tiles by itself (default_narrow)
-    int grid = 1;  // persistent CTAs
+    int n_few = 0;         // problems that take narrow tiles by default
+    int grid[2] = {1, 1};  // persistent CTAs of each part (batch_parts)
     int order = PSM_ORDER_DEPTH_FIRST;
-    // tile lists [wide / narrow tiles][order]
-    int n_items[4] = {0, 0, 0, 0};
-    DevBuf items[4];
+    // tile lists [kList*][order]
+    int n_items[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    DevBuf items[8];
     std::unique_ptr<psm::BatchParams> params;  // every problem's FwdParams (kernel argument)
     DevBuf counter, il_pos;
     cudaGraphExec_t exec = nullptr;
@@ -1951,10 +1952,30 @@ struct psm_batch {
 
 namespace {
 
-// The tile list of kernel K in the given order.
-template <class K>
-constexpr int item_list(int order) {
-    return 2 * (K::NX == kNarrowNX) + order;
+// Tile lists: every problem in wide or in narrow tiles, and, where the default takes both, the
+// problems of each.
+constexpr int kListWide = 0, kListNarrow = 1, kListWideOnly = 2, kListNarrowOnly = 3;
+
+// A batched run's launches: one for all problems, or, under the default variant, one for the
+// problems that take wide tiles and one for those that take narrow ones, so that a problem's
+// image does not depend on its company.  One grid, every problem in wide tiles and so: 3 problems of
+// 60 x 60 x 401 and 12 of 15 x 15 x 200 samples 0.92, 0.95 ms; one of 60 x 60 x 401 and 30 of
+// 25 x 28 x 300, which fill the GPU together, 1.11, 1.62 ms (psm_batch_autotune finds the wide
+// tiles there).
+struct BatchPart {
+    bool narrow;
+    int list;
+};
+int batch_parts(const psm_batch& b, BatchPart (&part)[2]) {
+    const int n = static_cast<int>(b.probs.size());
+    if (b.variant == PSM_FWD_DEFAULT && b.n_few > 0 && b.n_few < n) {
+        part[0] = {false, kListWideOnly};
+        part[1] = {true, kListNarrowOnly};
+        return 2;
+    }
+    const bool narrow = narrow_tiles(b.variant, b.store, b.kahan, b.n_few == n);
+    part[0] = {narrow, narrow ? kListNarrow : kListWide};
+    return 1;
 }
 
 template <class K>
@@ -1977,7 +1998,7 @@ static_assert(sizeof(psm::BatchItem) + sizeof(Job) <= kBatchStaticSmem, "s_item,
 // Shared-memory limit and persistent grid (resident CTAs on every SM) of the batch
 // kernel K; done before a stream capture, so the graph holds only the launch.
 template <class K>
-cudaError_t prepare_persistent(K, psm_batch& b) {
+cudaError_t prepare_persistent(K, psm_batch& b, const BatchPart& part, int i) {
     auto* kern = persistent_kernel<K>();
     const size_t smem = batch_smem<K>(b);
     cudaError_t e = allow_smem(kern, smem, kBatchStaticSmem);
@@ -1987,36 +2008,34 @@ cudaError_t prepare_persistent(K, psm_batch& b) {
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, b.ctx->device);
     if (e != cudaSuccess) return e;
-    b.grid = std::max(1, std::min(b.n_items[item_list<K>(b.order)], n_sm * std::max(per_sm, 1)));
+    b.grid[i] =
+        std::max(1, std::min(b.n_items[2 * part.list + b.order], n_sm * std::max(per_sm, 1)));
     return cudaSuccess;
 }
 
 template <class K>
-cudaError_t launch_persistent(K, const psm_batch& b, cudaStream_t s) {
-    const int w = item_list<K>(b.order);
-    persistent_kernel<K>()<<<b.grid, K::threads, batch_smem<K>(b), s>>>(
-        *b.params, b.items[w].as<psm::BatchItem>(), b.n_items[w], b.counter.as<int>(),
+cudaError_t launch_persistent(K, const psm_batch& b, const BatchPart& part, int i,
+                              cudaStream_t s) {
+    const int w = 2 * part.list + b.order;
+    persistent_kernel<K>()<<<b.grid[i], K::threads, batch_smem<K>(b), s>>>(
+        *b.params, b.items[w].as<psm::BatchItem>(), b.n_items[w], b.counter.as<int>() + i,
         b.ctx->err.as<int>());
     return cudaGetLastError();
 }
 
 // The one-grid kernel K (a CTA per tile of the list).
 template <class K>
-cudaError_t launch_items(K, const psm_batch& b, cudaStream_t s) {
-    const int w = item_list<K>(b.order);
+cudaError_t launch_items(K, const psm_batch& b, const BatchPart& part, cudaStream_t s) {
+    const int w = 2 * part.list + b.order;
     if (b.n_items[w] <= 0) return cudaSuccess;
     items_kernel<K>()<<<b.n_items[w], K::threads, batch_smem<K>(b), s>>>(
         *b.params, b.items[w].as<psm::BatchItem>());
     return cudaGetLastError();
 }
 
-// Tiles of a launch of every problem, and of one problem's own launch.
-bool batch_narrow(const psm_batch& b) {
-    return narrow_tiles(b.variant, b.store, b.kahan, b.few);
-}
+// Tiles of one problem's own launch.
 bool problem_narrow(const psm_batch& b, const BatchProblem& p) {
-    return narrow_tiles(b.variant, b.store, b.kahan,
-                        default_narrow(p.src.geom, static_cast<int64_t>(p.jobs.size())));
+    return narrow_tiles(b.variant, b.store, b.kahan, p.few);
 }
 
 // Repeated output rows of every problem (padded output inlines, main.cpp:268-285).
@@ -2033,26 +2052,30 @@ cudaError_t batch_copies(const psm_batch& b, cudaStream_t s) {
     return cudaSuccess;
 }
 
-// The work of one batched run, enqueued on s (persistent: counter and error word reset, one
-// launch, row copies).
+// The work of one batched run, enqueued on s (persistent: counters and error word reset, the
+// launches, row copies).
 cudaError_t batch_enqueue(psm_batch& b, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(b.ctx->err.p, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
-    if (b.mode == PSM_BATCH_ONE_GRID) {
-        e = with_kernel(b.amp, b.kahan, batch_narrow(b),
-                        [&](auto k) { return launch_items(k, b, s); });
-        if (e != cudaSuccess) return e;
-    } else if (b.mode == PSM_BATCH_PER_PROBLEM) {
+    BatchPart part[2];
+    const int n_parts = batch_parts(b, part);
+    if (b.mode == PSM_BATCH_PER_PROBLEM) {
         for (const BatchProblem& p : b.probs) {
             e = launch_fwd(p.P, static_cast<int>(p.jobs.size()), b.amp, problem_narrow(b, p), s,
                            b.kahan);
             if (e != cudaSuccess) return e;
         }
-    } else {
-        e = cudaMemsetAsync(b.counter.p, 0, sizeof(int), s);
+        return batch_copies(b, s);
+    }
+    if (b.mode == PSM_BATCH_PERSISTENT) {
+        e = cudaMemsetAsync(b.counter.p, 0, 2 * sizeof(int), s);
         if (e != cudaSuccess) return e;
-        e = with_kernel(b.amp, b.kahan, batch_narrow(b),
-                        [&](auto k) { return launch_persistent(k, b, s); });
+    }
+    for (int i = 0; i < n_parts; ++i) {
+        e = with_kernel(b.amp, b.kahan, part[i].narrow, [&](auto k) {
+            return b.mode == PSM_BATCH_ONE_GRID ? launch_items(k, b, part[i], s)
+                                                : launch_persistent(k, b, part[i], i, s);
+        });
         if (e != cudaSuccess) return e;
     }
     return batch_copies(b, s);
@@ -2069,20 +2092,21 @@ int batch_launch(psm_batch* b) {
             b->exec = nullptr;
         }
         // the kernels' shared-memory limits are set outside the capture
-        if (b->mode == PSM_BATCH_ONE_GRID)
-            PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
-                             using K = decltype(k);
-                             return allow_smem(items_kernel<K>(), batch_smem<K>(*b));
-                         }));
-        else if (b->mode == PSM_BATCH_PERSISTENT)
-            PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, batch_narrow(*b), [&](auto k) {
-                             return prepare_persistent(k, *b);
-                         }));
-        else
+        BatchPart part[2];
+        const int n_parts = batch_parts(*b, part);
+        if (b->mode == PSM_BATCH_PER_PROBLEM)
             for (bool narrow : {false, true})
                 PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, narrow, [&](auto k) {
                                  using K = decltype(k);
                                  return allow_smem(grid_kernel<K>(), batch_smem<K>(*b));
+                             }));
+        else
+            for (int i = 0; i < n_parts; ++i)
+                PSM_CUDA_TRY(c->st, with_kernel(b->amp, b->kahan, part[i].narrow, [&](auto k) {
+                                 using K = decltype(k);
+                                 return b->mode == PSM_BATCH_ONE_GRID
+                                            ? allow_smem(items_kernel<K>(), batch_smem<K>(*b))
+                                            : prepare_persistent(k, *b, part[i], i);
                              }));
         cudaGraph_t graph = nullptr;
         PSM_CUDA_TRY(c->st, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -2189,7 +2213,8 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
         max_inl = std::max(max_inl, max_inline_window(p.jobs_all));
         max_nt = std::max(max_nt, g.n_t);
         b->max_rows = std::max(b->max_rows, max_list_rows(p.jobs_all));
-        b->few = b->few && default_narrow(g, static_cast<int64_t>(p.jobs.size()));
+        p.few = default_narrow(g, static_cast<int64_t>(p.jobs.size()));
+        b->n_few += p.few;
     }
     if (!fits_staging(max_inl, max_nt, b->store == psm::kStoreF32 ? 8 : 4))
         return c->st.fail(PSM_ERR_UNSUPPORTED, "problems too large for one staging ring");
@@ -2273,12 +2298,16 @@ int psm_batch_create(psm_ctx* c, const psm_problem* problems, int n, psm_batch**
     //    the same tile one after another and the long tiles start early;
     //  * problem after problem, each in the grid kernel's order (crossline tile fastest,
     //    then output inline, then time tile, deepest first).
-    PSM_CUDA_TRY(c->st, b->counter.ensure(sizeof(int)));
-    for (int w = 0; w < 4; ++w) {
-        const int TT = psm::kTileT, NX = w < 2 ? kWideNX : kNarrowNX;
+    PSM_CUDA_TRY(c->st, b->counter.ensure(2 * sizeof(int)));
+    const bool mixed = b->n_few > 0 && b->n_few < n;
+    for (int w = 0; w < (mixed ? 8 : 4); ++w) {
+        const bool narrow = w / 2 == kListNarrow || w / 2 == kListNarrowOnly;
+        const bool only = w / 2 == kListWideOnly || w / 2 == kListNarrowOnly;
+        const int TT = psm::kTileT, NX = narrow ? kNarrowNX : kWideNX;
         std::vector<psm::BatchItem> items;
         for (int i = 0; i < n; ++i) {
             const BatchProblem& p = b->probs[i];
+            if (only && p.few != narrow) continue;
             const psm_geom& g = p.src.geom;
             for (int T0 = (g.n_t - 1) / TT * TT; T0 >= 0; T0 -= TT)
                 for (int j = 0; j < static_cast<int>(p.jobs.size()); ++j)
@@ -2353,7 +2382,8 @@ int psm_batch_set_variant(psm_batch* b, int variant) {
 
 int psm_batch_get_variant(psm_batch* b, int* variant) {
     if (!b || !variant) return PSM_ERR_ARG;
-    *variant = reported_variant(b->variant, b->store, b->kahan, b->few);
+    *variant = reported_variant(b->variant, b->store, b->kahan,
+                                b->n_few == static_cast<int>(b->probs.size()));
     return PSM_OK;
 }
 
@@ -2402,7 +2432,7 @@ int psm_batch_autotune(psm_batch* b, float* ms, int* best, int* best_order, int*
             cudaEventRecord(e1, c->stream);
             if ((rc = psm_batch_synchronize(b)) != PSM_OK) break;
             cudaEventElapsedTime(&t, e0, e1);
-            const bool narrow = batch_narrow(*b);
+            const bool narrow = narrow_tiles(cand, b->store, b->kahan, false);
             for (int v = 1; ms && v < PSM_FWD_N_VARIANTS; ++v)
                 if (effective_variant(v, b->store, b->kahan) == v &&
                     narrow_tiles(v, b->store, b->kahan, false) == narrow)

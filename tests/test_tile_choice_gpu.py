@@ -5,7 +5,7 @@ import dataclasses
 import numpy as np
 import pytest
 
-from poststackmig3d_b200 import Migrator
+from poststackmig3d_b200 import Batch, Migrator, Problem
 from poststackmig3d_b200 import synth as S
 from poststackmig3d_b200.shard import migrate_shard
 
@@ -81,3 +81,32 @@ def test_shards_are_the_whole_image(precision):
     for world in (2, 5):
         rows = [migrate_shard(g, W.data, W.vrms_cube(), r, world)[1] for r in range(world)]
         assert np.array_equal(np.concatenate(rows), whole)
+
+
+@pytest.mark.parametrize("precision,compensated", [("f32", False), ("bf16", True)])
+def test_batch_of_wide_and_narrow_problems(precision, compensated):
+    """Every problem of a batch takes the tiles that it takes by itself, whatever its company, in
+    every mode and order: the images are equal bit for bit."""
+    probs, singles = [], []
+    for k, (n_il, n_xl, n_t) in enumerate([(75, 5, 260), (20, 9, 300), (9, 3, 257),
+                                           (40, 30, 270), (16, 7, 130)]):
+        W = _workload(n_il, n_xl, n_t, pad_xl=k % 2, seed=30 + k)
+        g = dataclasses.replace(geometry_for(W), precision=precision, compensated=compensated)
+        with Migrator(0) as m:
+            _context(m, W, g)
+            singles.append(m.forward())
+            assert m.variant() == (WIDE if k in (0, 3) else NARROW)
+        probs.append(Problem(g, W.data, W.vrms_cube()))
+    with Migrator(0) as m, Batch(m, probs) as b:
+        for mode in (Batch.PERSISTENT, Batch.PER_PROBLEM, Batch.ONE_GRID):
+            for order in (Batch.DEPTH_FIRST, Batch.PROBLEM_ORDER):
+                b.set_mode(mode)
+                b.set_order(order)
+                for rep in range(2):  # capture, then replay of the graph
+                    b.run()
+                    for i, img in enumerate(singles):
+                        assert np.array_equal(b.image(i), img), (mode, order, rep, i)
+        b.set_variant(NARROW)  # one launch again
+        b.run()
+        assert np.array_equal(b.image(1), singles[1])
+        assert b.variant() == NARROW
