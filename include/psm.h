@@ -281,6 +281,12 @@ int psm_set_variant(psm_ctx *ctx, int variant);
  * geometry, for an id that 16-bit storage or compensated summation does not know the one it
  * stands for there. */
 int psm_get_variant(psm_ctx *ctx, int *variant);
+/* Nonzero: the ctx's forwards with fp32 storage add an output sample's terms in the order of its
+ * trace list (mirror distance, then crossline), as psm_lsm_cg's do, whatever the tiles.  For
+ * solvers around psm_forward / psm_forward_device: conjugate gradients carry a change of
+ * rounding in the operator into their step lengths.  0 (default): in the kernel's own order,
+ * which is up to 8% faster on small problems. */
+int psm_set_trace_order(psm_ctx *ctx, int on);
 /* Time one forward launch of each kernel on the resident cube (CUDA events on the ctx
  * stream), keep the fastest for this ctx.  ms[PSM_FWD_N_VARIANTS] (may be NULL) receives every
  * variant's kernel's time, ms[0] unused; *best (may be NULL) the chosen variant. */

@@ -112,6 +112,7 @@ _CUDA_SYMBOLS = [
     ("psm_lsm_cg", ctypes.c_int, [_P, _P, _P, ctypes.c_int, _P]),
     ("psm_set_variant", ctypes.c_int, [_P, ctypes.c_int]),
     ("psm_get_variant", ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int)]),
+    ("psm_set_trace_order", ctypes.c_int, [_P, ctypes.c_int]),
     ("psm_autotune", ctypes.c_int, [_P, _P, ctypes.POINTER(ctypes.c_int)]),
     ("psm_batch_create", ctypes.c_int, [_P, ctypes.POINTER(PsmProblem), ctypes.c_int,
                                         ctypes.POINTER(_P)]),

@@ -396,6 +396,7 @@ struct psm_ctx {
     int tail_nt = 0;        // samples per trace up to which `data` is written, and the bytes of
     size_t tail_bytes = 0;  // it whose rows' tails are known to be zero for that length
     bool few = false;       // narrow tiles by default (default_narrow)
+    bool trace_order = false;  // psm_set_trace_order
     // 16-bit storage: samples [n_il][n_xl][ns] and one scale per trace
     DevBuf words, scales;
     // adjoint: rows of each job (fold of duplicated output rows), image upload, job images
@@ -493,6 +494,13 @@ FwdParams volume_params(psm_ctx* c) {
 // Whether the ctx's forward launches use narrow tiles.
 bool ctx_narrow(const psm_ctx* c) {
     return narrow_tiles(c->variant, c->store, c->g.compensated != 0, c->few);
+}
+
+// The ctx's forward kernel on n_jobs jobs; ordered: terms added in trace order (fp32 storage).
+cudaError_t launch_ctx(const psm_ctx* c, const FwdParams& P, int n_jobs, cudaStream_t s,
+                       bool ordered) {
+    return launch_fwd(P, n_jobs, c->g.amp_correction != 0, ctx_narrow(c), s,
+                      c->g.compensated != 0, ordered && P.store == psm::kStoreF32);
 }
 
 // Host memory the CUDA driver copies through its own staging (not pinned or registered).
@@ -1024,9 +1032,8 @@ int psm_forward_async(psm_ctx* c) {
     cudaSetDevice(c->device);
     PSM_CUDA_TRY(c->st, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     FwdParams P = volume_params(c);
-    PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                   c->g.amp_correction != 0, ctx_narrow(c), c->stream,
-                                   c->g.compensated != 0));
+    PSM_CUDA_TRY(c->st, launch_ctx(c, P, static_cast<int>(c->jobs.size()), c->stream,
+                                   c->trace_order));
     // padded output inlines repeat the migrated edge inline (main.cpp:268-285)
     PSM_CUDA_TRY(c->st, copy_rows(c, c->image.as<float>(), c->stream));
     return PSM_OK;
@@ -1035,6 +1042,12 @@ int psm_forward_async(psm_ctx* c) {
 int psm_set_variant(psm_ctx* c, int variant) {
     if (!c || variant < 0 || variant >= PSM_FWD_N_VARIANTS) return PSM_ERR_ARG;
     c->variant = variant;
+    return PSM_OK;
+}
+
+int psm_set_trace_order(psm_ctx* c, int on) {
+    if (!c) return PSM_ERR_ARG;
+    c->trace_order = on != 0;
     return PSM_OK;
 }
 
@@ -1248,8 +1261,7 @@ int forward_waves(psm_ctx* c, const float* traces, const float* vrms, float* ima
             PSM_CUDA_TRY(c->st, cudaStreamWaitEvent(ks, ev[u], 0));
             FwdParams Q = P;
             Q.jobs = c->d_jobs_waves.as<Job>() + chunks[k].first;
-            PSM_CUDA_TRY(c->st, launch_fwd(Q, chunks[k].second, g.amp_correction != 0,
-                                           ctx_narrow(c), ks, g.compensated != 0));
+            PSM_CUDA_TRY(c->st, launch_ctx(c, Q, chunks[k].second, ks, c->trace_order));
             std::vector<int> out_rows;
             for (int t = 0; t < chunks[k].second; ++t) {
                 const int r = order[chunks[k].first + t].row;
@@ -1421,9 +1433,7 @@ int forward_dev(psm_ctx* c, const float* d_vec, float* d_img, bool ordered) {
     P.traces = d_vec;
     P.store = psm::kStoreF32;  // the operator pair of CG is the fp32 one
     P.image = d_img;
-    PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                   c->g.amp_correction != 0, ctx_narrow(c), c->stream,
-                                   c->g.compensated != 0, ordered));
+    PSM_CUDA_TRY(c->st, launch_ctx(c, P, static_cast<int>(c->jobs.size()), c->stream, ordered));
     PSM_CUDA_TRY(c->st, copy_rows(c, d_img, c->stream));
     return PSM_OK;
 }
@@ -1485,7 +1495,7 @@ int psm_forward_device(psm_ctx* c, const float* d_data, float* d_image) {
     PSM_CUDA_TRY(c->st, cudaMemcpy2DAsync(c->data.p, c->ns * sizeof(float), d_data,
                                           c->g.n_t * sizeof(float), c->g.n_t * sizeof(float),
                                           n_tr, cudaMemcpyDeviceToDevice, c->stream));
-    const int r = forward_dev(c, c->data.as<float>(), d_image, false);
+    const int r = forward_dev(c, c->data.as<float>(), d_image, c->trace_order);
     if (r) return r;
     c->have_traces = c->traces_readable = true;
     return PSM_OK;
@@ -1544,7 +1554,7 @@ int psm_lsm_cg(psm_ctx* c, const float* data, float* image, int iters, double* r
         psm::cg_alpha_kernel<<<1, 1, 0, s>>>(sc);                     // alpha = gamma / delta
         psm::cg_update_kernel<<<grid_for(nm + nd), 256, 0, s>>>(m, p, nm, r, q, nd, sc);
         if ((rc = dot_dev(c, r, r, nd, hist + k + 1))) return rc;     // ||r||^2
-        if ((rc = forward_dev(c, r, sv, true))) return rc;                  // s = M r
+        if ((rc = forward_dev(c, r, sv, true))) return rc;            // s = M r
         if ((rc = dot_dev(c, sv, sv, nm, sc + 2))) return rc;         // gamma_new
         psm::cg_beta_kernel<<<1, 1, 0, s>>>(sc);                      // beta, gamma
         psm::cg_direction_kernel<<<grid_for(nm), 256, 0, s>>>(p, sv, nm, sc);  // p = s + beta p
@@ -1874,9 +1884,8 @@ int psm_forward_streamed(psm_ctx* c, const psm_geom* g, const int32_t* out_cente
             float* img = c->str_img[k & 1].as<float>();
             FwdParams P = volume_params(c);
             P.image = img;
-            PSM_CUDA_TRY(c->st, launch_fwd(P, static_cast<int>(c->jobs.size()),
-                                           c->g.amp_correction != 0, ctx_narrow(c), c->stream,
-                                           c->g.compensated != 0));
+            PSM_CUDA_TRY(c->st, launch_ctx(c, P, static_cast<int>(c->jobs.size()), c->stream,
+                                           c->trace_order));
             PSM_CUDA_TRY(c->st, copy_rows(c, img, c->stream));  // padded inlines
             PSM_CUDA_TRY(c->st, cudaEventRecord(c->ev_done[k & 1], c->stream));
         }

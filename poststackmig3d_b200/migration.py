@@ -464,6 +464,11 @@ class Migrator:
         check(self._L.psm_get_variant(self._ctx, ctypes.byref(v)), self._err)
         return v.value
 
+    def set_trace_order(self, on: bool) -> None:
+        """Forwards with fp32 storage add terms in trace order, as lsm_cg's do
+        (psm_set_trace_order)."""
+        check(self._L.psm_set_trace_order(self._ctx, int(bool(on))), self._err)
+
     def autotune(self):
         """Time each forward kernel once on the resident cube and keep the fastest.
         Returns (best variant, {variant: its kernel's ms})."""

@@ -178,6 +178,7 @@ class _SlabOps:
 
     def __init__(self, lg: Geometry, vrms: np.ndarray, device: int):
         self.m = Migrator(device)
+        self.m.set_trace_order(True)  # Migrator.lsm_cg's operator
         self.m.set_geometry(lg)
         self.m.set_vrms(vrms)
 
@@ -327,6 +328,7 @@ class _DeviceSlabOps:
     def __init__(self, lg: Geometry, vrms: np.ndarray, device: int):
         import torch
         self.m = Migrator(device)
+        self.m.set_trace_order(True)  # Migrator.lsm_cg's operator
         self.m.set_geometry(lg)
         self.m.set_vrms(vrms)
         self.dev = torch.device(f"cuda:{device}")
