@@ -970,10 +970,19 @@ int psm_set_vrms_table(psm_ctx* c, const int32_t* p_il, const int32_t* p_xl,
     PSM_CUDA_TRY(c->st, upload(d_v, p_v, n_points, s));
     PSM_CUDA_TRY(c->st, upload(d_lil, il_labels, c->g.n_il, s));
     PSM_CUDA_TRY(c->st, upload(d_lxl, xl_labels, c->g.n_xl, s));
-    const size_t n_items = static_cast<size_t>(c->g.n_il) * c->g.n_xl *
-                           ((c->g.n_t + psm::kTableThreads - 1) / psm::kTableThreads);
-    const unsigned grid = static_cast<unsigned>(std::min<size_t>(n_items, 148 * 64));
-    psm::vrms_table_kernel<<<grid, psm::kTableThreads, 0, s>>>(
+    // work items of kTableThreads samples of a trace, unless they leave a third of the threads (a
+    // fifth, for a table of fewer points) without samples or the table has next to no points.  Whole
+    // calls, by items and by the flat kernel: 300 x 300 x 20 samples, 54 points 0.51, 0.23 ms; 200 x
+    // 200 x 130, 54 points 0.67, 0.56, 1 point 0.118, 0.085; x 300, 6 points 0.244, 0.229; x 270, 60
+    // points 1.11, 1.18; x 400, 60 points 1.64, 1.72
+    const size_t n_tr = static_cast<size_t>(c->g.n_il) * c->g.n_xl;
+    const int n_seg = (c->g.n_t + psm::kTableThreads - 1) / psm::kTableThreads;
+    const int64_t held = static_cast<int64_t>(n_seg) * psm::kTableThreads;
+    const bool flat = 2 * held > 3LL * c->g.n_t || n_points < 4 ||
+                      (n_points < 40 && 4 * held > 5LL * c->g.n_t);
+    const unsigned grid = static_cast<unsigned>(std::min<size_t>(n_tr * n_seg, 148 * 64));
+    auto* kern = flat ? psm::vrms_table_flat_kernel : psm::vrms_table_kernel;
+    kern<<<flat ? vrms_blocks(n_tr * c->g.n_t) : grid, flat ? 256 : psm::kTableThreads, 0, s>>>(
         d_il.as<int32_t>(), d_xl.as<int32_t>(), d_t.as<double>(), d_v.as<float>(), n_points,
         vmin, d_lil.as<int32_t>(), d_lxl.as<int32_t>(), c->g.n_il, c->g.n_xl, c->g.n_t,
         c->g.dt_seconds, c->vrms.as<float>());

@@ -37,6 +37,28 @@ __device__ __forceinline__ float root_to_float(double x, bool* sure) {
     return __double2float_rn(s);
 }
 
+// One table point's share of the weighted sums, at squared distance x: with the fast root (*sure as
+// above), and with the exact one, which is true for an exact hit.
+__device__ __forceinline__ void blend_fast(double x, float v, float& sv, float& sw, bool* sure) {
+    const float w = __frcp_rn(__fadd_rn(1.0f, root_to_float(x, sure)));
+    sv = __fadd_rn(sv, __fmul_rn(v, w));
+    sw = __fadd_rn(sw, w);
+}
+__device__ __forceinline__ bool blend_exact(double x, float v, float& sv, float& sw) {
+    const double d = __dsqrt_rn(x);
+    if (d < 1e-10) return true;
+    const float w = __fdiv_rn(1.0f, __fadd_rn(1.0f, __double2float_rn(d)));
+    sv = __fadd_rn(sv, __fmul_rn(v, w));
+    sw = __fadd_rn(sw, w);
+    return false;
+}
+__device__ __forceinline__ float blend_result(bool hit, float hit_v, float sv, float sw,
+                                              float vmin) {
+    if (hit) return hit_v;
+    const float r = sw > 0.0f ? __fdiv_rn(sv, sw) : vmin;
+    return r <= 0.0f ? vmin : r;
+}
+
 // Text-table Vrms: every point (il, xl, time, v) weighted by 1 / (1 + dist) with dist mixing
 // label units and seconds; an exact hit (dist < 1e-10) returns that point's v; a result <= 0
 // (or no weight) gives vmin.  out [n_il][n_xl][n_t], t0 = t * dt.
@@ -81,10 +103,7 @@ vrms_table_kernel(const int32_t* __restrict__ p_il, const int32_t* __restrict__ 
             for (int p = 0; p < cnt; ++p) {
                 const double2 u = at[p];
                 const double c = __dsub_rn(u.y, time);
-                const float d = root_to_float(__dadd_rn(u.x, __dmul_rn(c, c)), &sure);
-                const float w = __frcp_rn(__fadd_rn(1.0f, d));
-                sv = __fadd_rn(sv, __fmul_rn(vel[p], w));
-                sw = __fadd_rn(sw, w);
+                blend_fast(__dadd_rn(u.x, __dmul_rn(c, c)), vel[p], sv, sw, &sure);
             }
             if (sure) continue;
             sv = v0;  // again, with the exact root
@@ -93,24 +112,50 @@ vrms_table_kernel(const int32_t* __restrict__ p_il, const int32_t* __restrict__ 
             for (int p = 0; p < cnt; ++p) {
                 const double2 u = at[p];
                 const double c = __dsub_rn(u.y, time);
-                const double d = __dsqrt_rn(__dadd_rn(u.x, __dmul_rn(c, c)));
-                if (d < 1e-10) {
+                if (blend_exact(__dadd_rn(u.x, __dmul_rn(c, c)), vel[p], sv, sw)) {
                     hit = true;
                     hit_v = vel[p];
                     break;
                 }
-                const float w = __fdiv_rn(1.0f, __fadd_rn(1.0f, __double2float_rn(d)));
-                sv = __fadd_rn(sv, __fmul_rn(vel[p], w));
-                sw = __fadd_rn(sw, w);
             }
         }
         if (t >= n_t) continue;
-        float r = hit_v;
-        if (!hit) {
-            r = sw > 0.0f ? __fdiv_rn(sv, sw) : vmin;
-            if (r <= 0.0f) r = vmin;
+        out[tr * n_t + t] = blend_result(hit, hit_v, sv, sw, vmin);
+    }
+}
+
+// The same for a table of few points or traces that leave a work item's threads without samples: a
+// thread per sample, which reads the points from global memory and sums their label parts itself.
+__global__ void vrms_table_flat_kernel(const int32_t* __restrict__ p_il,
+                                       const int32_t* __restrict__ p_xl,
+                                       const double* __restrict__ p_time,
+                                       const float* __restrict__ p_v, int n_points, float vmin,
+                                       const int32_t* __restrict__ il,
+                                       const int32_t* __restrict__ xl, int n_il, int n_xl,
+                                       int n_t, double dt, float* __restrict__ out) {
+    const int64_t n = static_cast<int64_t>(n_il) * n_xl * n_t;
+    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
+         k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t tr = k / n_t;
+        const int32_t a_il = il[tr / n_xl], a_xl = xl[tr % n_xl];
+        const double time = __dmul_rn(static_cast<double>(static_cast<int>(k - tr * n_t)), dt);
+        auto square = [&](int p) {
+            const double a = fabs(static_cast<double>(p_il[p] - a_il));
+            const double b = fabs(static_cast<double>(p_xl[p] - a_xl));
+            const double c = __dsub_rn(p_time[p], time);
+            return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
+        };
+        float sv = 0.0f, sw = 0.0f, hit_v = 0.0f;
+        bool hit = false, sure = true;
+        for (int p = 0; p < n_points; ++p) blend_fast(square(p), p_v[p], sv, sw, &sure);
+        if (!sure) {  // again, with the exact root
+            sv = sw = 0.0f;
+            for (int p = 0; p < n_points && !hit; ++p) {
+                hit = blend_exact(square(p), p_v[p], sv, sw);
+                if (hit) hit_v = p_v[p];
+            }
         }
-        out[tr * n_t + t] = r;
+        out[k] = blend_result(hit, hit_v, sv, sw, vmin);
     }
 }
 
