@@ -247,8 +247,8 @@ int psm_adjoint_device(psm_ctx *ctx, const float *d_image, float *d_data);
 /* Least-squares migration: `iters` iterations of CG (CGLS) on min ||M^T m - data||^2 from
  * m = 0, with FP32 operators and FP64 inner products and step lengths computed on the GPU.
  * data [n_il][n_xl][n_t] (host) in, image [n_oi][n_ox][n_t] (host) out, resid[iters + 1]
- * (host, may be NULL) the data-residual norms ||M^T m_k - data||.  Overwrites the resident
- * traces. */
+ * (host, may be NULL) the data-residual norms ||M^T m_k - data||.  Afterwards the ctx has no
+ * resident traces. */
 int psm_lsm_cg(psm_ctx *ctx, const float *data, float *image, int iters, double *resid);
 
 /* Forward-kernel variants.  There are two kernels, which differ in the output crosslines of a
@@ -372,7 +372,9 @@ int psm_batch_count_terms(psm_batch *batch, int64_t *n_terms);
  * output_slice flat [n_out_xl][n_t] instead of vector<vector<float>>; xl_pos_indices is
  * unused (as in the reference) and may be NULL.  Uploads the buffer on each call, so it is
  * the slow path; the resident-cube calls above are the fast path.  Thread-safe: each host
- * thread gets its own device staging. */
+ * thread gets its own device staging.  t0_times may be in any order.  The call chooses its
+ * tiles by its own size, so its output equals the inline's rows of a whole-cube migration to
+ * FP32 rounding (the order of an output sample's sum), not always bit for bit. */
 int psm_kirchhoff_inline(const float *input_buffer, size_t n_buf_il, size_t n_buf_xl,
                          size_t n_t, const float *velocity_slice, float *output_slice,
                          size_t n_out_xl, const int32_t *il_pos_indices,

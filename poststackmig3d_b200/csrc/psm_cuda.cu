@@ -1486,8 +1486,9 @@ int psm_adjoint_async(psm_ctx* c) {
     PSM_CUDA_TRY(c->st, cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     int r = adjoint_dev(c, c->image.as<float>(), c->data.as<float>());
     if (r) return r;
-    c->have_traces = false;      // the staged storage still holds the earlier traces
-    c->traces_readable = true;   // the fp32 cube holds M^T image
+    // the fp32 cube holds M^T image; 16-bit storage still holds the earlier traces
+    c->have_traces = false;
+    c->traces_readable = true;
     return PSM_OK;
 }
 
@@ -1574,7 +1575,7 @@ int psm_lsm_cg(psm_ctx* c, const float* data, float* image, int iters, double* r
     PSM_CUDA_TRY(c->st, cudaMemcpyAsync(h.data(), hist, (iters + 1) * sizeof(double),
                                         cudaMemcpyDeviceToHost, s));
     PSM_CUDA_TRY(c->st, cudaStreamSynchronize(s));
-    c->have_traces = c->traces_readable = false;  // the cube now holds the last residual
+    c->have_traces = c->traces_readable = false;  // (a forward wants its traces uploaded again)
     if (resid)
         for (int k = 0; k <= iters; ++k) resid[k] = std::sqrt(std::max(h[k], 0.0));
     return read_device_error(c);
