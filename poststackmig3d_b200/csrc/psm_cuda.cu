@@ -199,6 +199,10 @@ template <class K>
 auto grid_kernel() {
     return psm::fwd_kernel<K::AMP, K::KAHAN, K::ORDERED, K::NX, K::CAP, K::MINB>;
 }
+template <class K>
+auto pairs_kernel() {
+    return psm::fwd_pairs_kernel<K::AMP, K::NX, K::CAP, K::MINB>;
+}
 
 // Lets a kernel be launched with `smem` bytes of dynamic shared memory.  The limit belongs to the
 // kernel, which other host threads launch with other amounts, so it is set to the same value on
@@ -212,8 +216,8 @@ cudaError_t allow_smem(Kernel* kern, size_t smem, size_t fixed = 0) {
 }
 
 template <class K>
-cudaError_t launch_grid(K, const FwdParams& P, int n_jobs, cudaStream_t s) {
-    auto* kern = grid_kernel<K>();
+cudaError_t launch_grid(K, void (*kern)(const FwdParams), const FwdParams& P, int n_jobs,
+                        cudaStream_t s) {
     const size_t smem = K::Layout::total(P.store, P.max_rows);
     if (n_jobs > 65535) return cudaErrorInvalidValue;  // grid y
     dim3 grid((P.n_ox + K::NX - 1) / K::NX, n_jobs, (P.n_t + psm::kTileT - 1) / psm::kTileT);
@@ -232,7 +236,11 @@ cudaError_t launch_grid(K, const FwdParams& P, int n_jobs, cudaStream_t s) {
 cudaError_t launch_fwd(const FwdParams& P, int n_jobs, bool amp, bool narrow, cudaStream_t s,
                        bool kahan = false, bool ordered = false) {
     if (n_jobs <= 0 || P.n_ox <= 0 || P.n_t <= 0) return cudaSuccess;
-    auto f = [&](auto k) { return launch_grid(k, P, n_jobs, s); };
+    auto f = [&](auto k) { return launch_grid(k, grid_kernel<decltype(k)>(), P, n_jobs, s); };
+    if (P.store == psm::kStorePairs)  // (fp32 sums without compensation only)
+        return with_kernel(amp, false, narrow, [&](auto k) {
+            return launch_grid(k, pairs_kernel<decltype(k)>(), P, n_jobs, s);
+        });
     return ordered ? with_kernel<true>(amp, kahan, narrow, f)
                    : with_kernel(amp, kahan, narrow, f);
 }

@@ -64,7 +64,7 @@ struct FwdStage {
 // one mirror buffer for all stages, so that as many CTAs fit an SM as with fp32 traces: the
 // producer waits for the folder to be done with it, which it is long before the consumers
 // release a stage.  (psm_forward_noalloc, 101 x 101 x 501 samples: 2.71 ms with a buffer per stage,
-// which leaves room for one CTA of the wide tiles, 2.04 ms so.)
+// which leaves room for one CTA of the wide tiles, 1.91 ms so.)
 template <int NX, int CAP>
 struct FwdLayout {
     static_assert(NX % 2 == 0 && CAP % 8 == 0, "crossline pairs; 16-byte aligned windows");
@@ -78,16 +78,13 @@ struct FwdLayout {
     static constexpr unsigned kRing = (kBlk + 8 * 32 + 127) & ~127u;
     static constexpr unsigned kStageBytes = 8u * CAP;
     static constexpr unsigned kMirror = kRing + kStages * kStageBytes;
-    // bytes from one stage's mirror buffer to the next
-    static __host__ __device__ constexpr unsigned mirror_step(int store) {
-        return store == kStorePairs ? 0u : static_cast<unsigned>(CAP) * store_bytes(store);
-    }
-    static __host__ __device__ constexpr unsigned rows(int store) {
-        return kMirror + (store == kStorePairs ? 8u * CAP : kStages * mirror_step(store));
+    // the row tables, for raw samples of rb bytes
+    static __host__ __device__ constexpr unsigned rows_at(int rb) {
+        return kMirror + (rb == 8 ? 1 : kStages) * static_cast<unsigned>(CAP) * rb;
     }
     // row tables: running slot counts and dx^2
     static __host__ __device__ constexpr unsigned total(int store, int max_rows) {
-        return rows(store) + 4u * (2u * static_cast<unsigned>(max_rows) + 1u);
+        return rows_at(store_bytes(store)) + 4u * (2u * static_cast<unsigned>(max_rows) + 1u);
     }
     static_assert(kTab % 16 == 0 && sizeof(FwdStage<NX>) % 16 == 0, "16-byte aligned tables");
 };
@@ -281,10 +278,12 @@ struct False {
 // partial, and the partials are added to the accumulator with Kahan's compensation, so the long
 // sum over the aperture carries no growing rounding error.
 //
+// PAIRS: caller-made pairs (kStorePairs), else any other storage.
+//
 // All warps of the CTA call fwd_tile; `it` counts the ring stages the CTA has used, so that
 // consecutive tiles of a persistent CTA continue the ring's phases (every stage, the
 // end-of-stream marker included, is released).  Returns false when a bounded wait expired.
-template <bool AMP, bool KAHAN, bool ORDERED, int NX, int CAP>
+template <bool AMP, bool KAHAN, bool ORDERED, int NX, int CAP, bool PAIRS = false>
 __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int x0, int T0,
                                          unsigned char* smem, uint32_t& it) {
     using L = FwdLayout<NX, CAP>;
@@ -359,8 +358,8 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
     }
     // The producer's share of the wait: smallest and largest t0 of each block of 32 samples (lane
     // b holds block b), whatever their order (the per-inline call takes the caller's times).
-    // A sample has terms only with t0 > 0; every other counts as 0.  (Not unrolled: 8.84 against
-    // 8.81 ms, 133 x 87 x 733 samples.)
+    // A sample has terms only with t0 > 0; every other counts as 0.  (Unrolled, the loop moves the
+    // evaluation loops: 8.86 against 8.84 ms, 133 x 87 x 733 samples.)
     float t0min = 0.0f, t0max = 0.0f;
     if (warp == 0) {
 #pragma unroll 1
@@ -379,7 +378,8 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        const int store = P.store, rb = store_bytes(store);
+        const int store = PAIRS ? kStorePairs : P.store;
+        const int rb = PAIRS ? 8 : store == kStoreF32 ? 4 : 2;
         const int A = store == kStoreBF16 || store == kStoreF16 ? 8 : 4;  // window alignment
         // bounds of each block of 32 samples over the tile's crosslines, in two float4: (largest
         // B, smallest t0, 2 / (v_max tan), 4 / v_max^2), (largest t0^2, 4 / v_min^2, largest t0^2
@@ -416,7 +416,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
         const int xa = max(x0 + P.xoff, 0);
         const int xb = min(min(x0 + NX, P.n_ox) - 1 + P.xoff,
                            P.compat_pad ? 0x3fffffff : P.n_vx - 1);
-        int* row_pre = reinterpret_cast<int*>(smem + L::rows(store));
+        int* row_pre = reinterpret_cast<int*>(smem + L::rows_at(rb));
         float* row_dx2 = reinterpret_cast<float*>(row_pre + P.max_rows + 1);
         const int n_inl = max(job.i1 - job.i0, 0);
         // rows of the trace list: the buffer inlines, or the mirror distances d from the centre
@@ -558,7 +558,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                 const int stage = it % kStages;
                 const uint32_t par = ((it / kStages) & 1u) ^ 1u;
                 int ok = lane == 0 ? mbar_wait(&empty[stage], par, P.err, P.wait_us) : 0;
-                if (lane == 0 && ok && store == kStorePairs && it > it_begin)  // the mirror buffer
+                if (PAIRS && lane == 0 && ok && it > it_begin)  // the mirror buffer
                     ok = mbar_wait(&ready[(it - 1) % kStages], ((it - 1) / kStages) & 1u, P.err,
                                    P.wait_us);
                 if (!__shfl_sync(0xffffffffu, ok, 0)) {
@@ -578,7 +578,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
                     store == kStoreF32 ? L::kRing + stage * L::kStageBytes + 4u * (tot + off)
                                        : dst + (8u - rb) * copy;
                 const uint32_t dst_mir =
-                    L::kMirror + static_cast<uint32_t>(stage) * L::mirror_step(store) + off * rb;
+                    L::kMirror + ((PAIRS ? 0u : static_cast<uint32_t>(stage) * CAP) + off) * rb;
                 const int slot = __popc(slots & ((1u << lane) - 1u));
                 if (mine) {
                     m.base[slot] = static_cast<int>(dst - 8u * ws - 0x58000000u);
@@ -653,7 +653,7 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
 
     if (warp == 1) {
         // ---------------------------------------------------------------- folder
-        const int store = P.store;
+        const int store = PAIRS ? kStorePairs : P.store;
         bool alive = true;
         while (true) {
             const int stage = it % kStages;
@@ -673,12 +673,12 @@ __device__ __forceinline__ bool fwd_tile(const FwdParams& P, const Job job, int 
             } else if (!ORDERED) {
                 for (int g = 0; g < n; ++g) {
                     const int4 w = m.win[g];
-                    if (store == kStoreBF16)
-                        fold_window<kStoreBF16>(smem, w.x, w.y, w.z, m.scale[g], lane);
-                    else if (store == kStoreF16)
-                        fold_window<kStoreF16>(smem, w.x, w.y, w.z, m.scale[g], lane);
-                    else
+                    if constexpr (PAIRS)
                         fold_window<kStorePairs>(smem, w.x, w.y, w.z, make_float2(0.f, 0.f), lane);
+                    else if (store == kStoreBF16)
+                        fold_window<kStoreBF16>(smem, w.x, w.y, w.z, m.scale[g], lane);
+                    else
+                        fold_window<kStoreF16>(smem, w.x, w.y, w.z, m.scale[g], lane);
                 }
             }
             fence_async_smem();  // the next fill of this stage is the async proxy's
@@ -930,6 +930,17 @@ __global__ void __launch_bounds__(32 * (NX + 2), MINB) fwd_kernel(const FwdParam
     fwd_tile<AMP, KAHAN, ORDERED, NX, CAP>(P, P.jobs[blockIdx.y], blockIdx.x * NX,
                                            static_cast<int>(gridDim.z - 1 - blockIdx.z) * kTileT,
                                            smem_raw, it);
+}
+
+// The same on caller-made pairs, a kernel of its own, so that the others carry none of it.
+template <bool AMP, int NX, int CAP, int MINB>
+__global__ void __launch_bounds__(32 * (NX + 2), MINB) fwd_pairs_kernel(const FwdParams P) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    if (threadIdx.x == 0) ring_init<NX, CAP>(smem_raw);
+    uint32_t it = 0;
+    fwd_tile<AMP, false, false, NX, CAP, true>(
+        P, P.jobs[blockIdx.y], blockIdx.x * NX,
+        static_cast<int>(gridDim.z - 1 - blockIdx.z) * kTileT, smem_raw, it);
 }
 
 // Parameters of every problem of a batched launch, passed by value: they live in the
