@@ -2602,7 +2602,9 @@ int psm_kirchhoff_inline(const float* input_buffer, size_t n_buf_il, size_t n_bu
                         std::string(#call) + ": " + cudaGetErrorString(e_));                \
     } while (0)
     if (S->device != dev || !S->stream) {
-        S->host.release();  // (its events belong to the device)
+        S->host.release();  // (its events, and the workspaces, belong to the device)
+        for (DevBuf* b : {&S->data, &S->vel, &S->out, &S->job, &S->il_pos, &S->t0, &S->err})
+            b->release();
         if (S->stream) cudaStreamDestroy(S->stream);
         S->stream = nullptr;
         PSM_INL_TRY(cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking));
